@@ -105,7 +105,7 @@ int32_t zkb_basefold_encode(zkb_ctx* c, const uint32_t* coeffs, size_t n, int32_
         const u32* d = on_device ? coeffs : up_pad(c, coeffs, n, n);
         BfTables tb = bf_tables(c, log_n);
         u32* cw = out_on_device ? codeword : (u32*)c->scratch(2 * n_pad * 4);
-        bf_encode(c, CoefSrc{d, 1, (u32)n, log_n}, log_n, tb, cw);
+        bf_encode(c, CoefSrc{d, 1, (u32)n, log_n}, log_n, tb, cw, true);
         if (!out_on_device) ZKB_CUDA(cudaMemcpyAsync(codeword, cw, 2 * n_pad * 4, cudaMemcpyDeviceToHost, c->stream));
         ZKB_CUDA(cudaStreamSynchronize(c->stream));
         c->scratch_reset();

@@ -12,11 +12,14 @@
 
 namespace zkb {
 
+// Words of a buffer that bfb_lincomb_kernel reads or writes for `len` values: whole 16-byte vectors.
+inline size_t bfb_vec_len(size_t len) { return len < 4 ? 4 : len; }
 __global__ void bfb_coeffs_kernel(const u32* __restrict__ rho, u32 k, u32* coef) {        // [1, rho, rho^2, ...] (:1239-1242)
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) coef[i] = pow31(rho[0], i);
 }
-// out[j] = sum_{i in [first, first + count)} coef[i] * cws[i][j], j < len.  Codewords and out are cudaMalloc'd and len is a power of
-// two >= 4 (a codeword has 2 * 2^log_n >= 4 words), so every thread moves 16-byte vectors; the codewords are read once (evict first).
+// out[j] = sum_{i in [first, first + count)} coef[i] * cws[i][j], j < len.  Of every codeword [v || v] only v is kept and summed.
+// The buffers are cudaMalloc'd and len is a power of two >= 2 that fills whole 16-byte vectors (a lone polynomial of two coefficients
+// has its buffers padded to four words); the codewords are read once (evict first).
 __global__ void __launch_bounds__(256) bfb_lincomb_kernel(const u32* const* __restrict__ cws, const u32* __restrict__ coef, u32 first, u32 count,
                                                           size_t len, u32* __restrict__ out) {
     const size_t n4 = len >> 2;
@@ -57,9 +60,10 @@ __global__ void __launch_bounds__(256) bfb_open_kernel(const u32* __restrict__ v
                                                        u32 tree_half, u32* out) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const size_t pw = 2 + 4 * (size_t)(h - 1);
+    // values and nodes are one half of the codeword and the tree over it (height h - 1)
     for (u32 item = warp; item < 2 * BF_QUERIES; item += nwarps) {
         const size_t pos = (size_t)(idx[item >> 1] & (tree_half - 1)) + ((item & 1) ? tree_half : 0);
-        mk_gather_path(values, size_t(1) << h, nodes, h, pos, out + item * pw, lane, 32);
+        mk_gather_path_doubled(values, nodes, h - 1, pos, out + item * pw, lane, 32);
     }
 }
 __global__ void bfb_final_value_kernel(const u32* __restrict__ coef, const u32* __restrict__ evals, u32 k, u32* out) {
@@ -121,16 +125,17 @@ BfbPending bfb_enqueue(zkb_bf_batch* B, TrState* tr, bool individual) {
         groups.push_back(Group{B->e[gs].log_n, gs, ge});
         gs = ge;
     }
-    const size_t cw_len0 = size_t(2) << log_n;
-    u32* cw0 = (u32*)c->scratch(cw_len0 * 4);
-    uint4* tree0 = (uint4*)c->scratch(mk_node_count(log_n + 1) * 16 + 16);
-    bfb_lincomb_kernel<<<grid_for(c, cw_len0 / 4), 256, 0, c->stream>>>(B->cw_ptrs_dev, coef, groups[0].s, groups[0].e - groups[0].s, cw_len0, cw0);
+    const size_t cw_len0 = size_t(1) << log_n;                 // the batched codeword is [v || v] like its parts
+    u32* cw0 = (u32*)c->scratch(cw_len0 * 4 + 16);
+    uint4* tree0 = (uint4*)c->scratch(mk_node_count(log_n) * 16 + 16);
+    bfb_lincomb_kernel<<<grid_for(c, bfb_vec_len(cw_len0) / 4), 256, 0, c->stream>>>(B->cw_ptrs_dev, coef, groups[0].s, groups[0].e - groups[0].s, bfb_vec_len(cw_len0), cw0);
     ZKB_LAUNCHED(c);
     MkFold none{};
-    mk_build(c, kind, MK_VALUES, cw0, cw_len0, log_n + 1, tree0, none);
+    none.doubled = 1;
+    mk_build(c, kind, MK_VALUES, cw0, cw_len0, log_n, tree0, none);
     u32* fold_point = (u32*)c->scratch(((size_t)log_n + 1) * 4);
     pd.batched_root_off = c->rec_alloc(4);
-    bfb_begin_kernel<<<1, 1, 0, c->stream>>>(tr, tree0 + mk_layer_offset(log_n + 1, log_n + 1), log_n, fold_point, c->rec_dev + pd.batched_root_off);
+    bfb_begin_kernel<<<1, 1, 0, c->stream>>>(tr, tree0 + mk_node_count(log_n), log_n, fold_point, c->rec_dev + pd.batched_root_off);
     ZKB_LAUNCHED(c);
 
     const bool in_order = c->opt_bf_in_order || c->capturing;
@@ -155,17 +160,20 @@ BfbPending bfb_enqueue(zkb_bf_batch* B, TrState* tr, bool individual) {
         const u32 h_prev = log_n + 1 - round;
         const size_t half = size_t(1) << (h_prev - 1);           // length of the folded codeword
         const u32 fold_level = log_n - 1 - round, target = log_n - 1 - round;
-        u32* next_cw = (u32*)c->scratch(half * 4 + 16);
-        uint4* next_tree = (uint4*)c->scratch(mk_node_count(h_prev - 1) * 16 + 16);
+        // the first fold leaves the codeword's half as it is (see basefold.cuh): without a codeword that joins there it is reused
+        const bool reuse = round == 0 && !(next_group < groups.size() && groups[next_group].log_n == target);
+        u32* next_cw = reuse ? cw0 : (u32*)c->scratch(half * 4 + 16);
+        uint4* next_tree = reuse ? tree0 : (uint4*)c->scratch(mk_node_count(h_prev - 1) * 16 + 16);
         MkFold f{};
         f.prev = prev_cw; f.out = next_cw;
         f.weights = tb.w_flat + ((size_t(1) << fold_level) - 1);
         f.w_len = size_t(1) << fold_level;
+        f.prev_partner = round == 0 ? 0 : half;
         f.alpha = fold_point + round;
         c->stream = work;
         try {
             // codewords that reach their own length at this round join the chain (:1304-1314); a codeword of 2 * 2^target values
-            // is exactly as long as the folded one
+            // is exactly as long as the folded one, and its two halves are the same
             u32 first = 0, count = 0;
             while (next_group < groups.size() && groups[next_group].log_n == target) {
                 if (!count) first = groups[next_group].s;
@@ -173,12 +181,14 @@ BfbPending bfb_enqueue(zkb_bf_batch* B, TrState* tr, bool individual) {
                 next_group++;
             }
             if (count) {
-                u32* add = (u32*)c->scratch(half * 4 + 16);
-                bfb_lincomb_kernel<<<grid_for(c, half / 4 ? half / 4 : 1), 256, 0, c->stream>>>(B->cw_ptrs_dev, coef, first, count, half, add);
+                u32* add = (u32*)c->scratch(half / 2 * 4 + 16);
+                const size_t len = bfb_vec_len(half / 2);
+                bfb_lincomb_kernel<<<grid_for(c, len / 4), 256, 0, c->stream>>>(B->cw_ptrs_dev, coef, first, count, len, add);
                 ZKB_LAUNCHED(c);
                 f.add = add;
+                f.add_mask = half / 2 - 1;
             }
-            mk_build(c, kind, MK_FOLD, nullptr, half, h_prev - 1, next_tree, f);
+            if (!reuse) mk_build(c, kind, MK_FOLD, nullptr, half, h_prev - 1, next_tree, f);
             c->stream = main_stream;
             if (!in_order) {
                 ZKB_CUDA(cudaEventRecord(c->side_event(round), work));
@@ -189,6 +199,7 @@ BfbPending bfb_enqueue(zkb_bf_batch* B, TrState* tr, bool individual) {
             rp.alpha_next = round + 1 < log_n ? fold_point + log_n : nullptr;    // the value is already in fold_point; the slot behind it takes the copy
             rp.prev_values = prev_cw; rp.prev_nodes = prev_tree; rp.fold_values = next_cw; rp.fold_nodes = next_tree;
             rp.h_prev = h_prev;
+            rp.prev_doubled = round == 0;
             const size_t off = c->rec_alloc(bf_round_words(h_prev));
             rp.rec = c->rec_dev + off;
             pd.round_off.push_back(off);
@@ -273,14 +284,16 @@ int32_t zkb_basefold_batch_precommit(zkb_ctx* c, const uint32_t* const* coeffs, 
                     if (e.n) ZKB_CUDA(cudaMemcpyAsync(d, coeffs[idx], e.n * 4, cudaMemcpyHostToDevice, c->stream));
                     e.coeffs = d;
                 }
-                ZKB_CUDA(cudaMalloc(&e.cw, 2 * n_pad * 4));
+                ZKB_CUDA(cudaMalloc(&e.cw, bfb_vec_len(n_pad) * 4));
                 B->owned.push_back(e.cw);
-                ZKB_CUDA(cudaMalloc(&e.tree, mk_node_count(e.log_n + 1) * 16 + 16));
+                if (n_pad < 4) ZKB_CUDA(cudaMemsetAsync(e.cw, 0, 16, c->stream));
+                ZKB_CUDA(cudaMalloc(&e.tree, mk_node_count(e.log_n) * 16 + 16));
                 B->owned.push_back(e.tree);
-                bf_encode(c, CoefSrc{e.coeffs, 1, (u32)e.n, e.log_n}, e.log_n, tb, e.cw);
+                bf_encode(c, CoefSrc{e.coeffs, 1, (u32)e.n, e.log_n}, e.log_n, tb, e.cw, false);
                 MkFold none{};
-                mk_build(c, node_hash, MK_VALUES, e.cw, 2 * n_pad, e.log_n + 1, e.tree, none);
-                ZKB_CUDA(cudaMemcpyAsync(e.root, e.tree + mk_layer_offset(e.log_n + 1, e.log_n + 1), 16, cudaMemcpyDeviceToHost, c->stream));
+                none.doubled = 1;
+                mk_build(c, node_hash, MK_VALUES, e.cw, n_pad, e.log_n, e.tree, none);
+                ZKB_CUDA(cudaMemcpyAsync(e.root, e.tree + mk_node_count(e.log_n), 16, cudaMemcpyDeviceToHost, c->stream));
                 B->e.push_back(e);
                 ptrs.push_back(e.cw);
             }
@@ -314,7 +327,7 @@ void zkb_basefold_batch_destroy(zkb_bf_batch* B) {
 size_t zkb_basefold_batch_count(const zkb_bf_batch* B) { return B ? B->e.size() : 0; }
 uint64_t zkb_basefold_batch_device_bytes(const zkb_bf_batch* B) {
     uint64_t t = 0;
-    if (B) for (auto& e : B->e) t += (uint64_t(8) << e.log_n) + (mk_node_count(e.log_n + 1) * 16 + 16);
+    if (B) for (auto& e : B->e) t += zkb::bfb_vec_len(size_t(1) << e.log_n) * 4 + (mk_node_count(e.log_n) * 16 + 16);
     return t;
 }
 

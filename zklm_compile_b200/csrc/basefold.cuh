@@ -8,9 +8,14 @@
 //   opening     per round: alpha, fold coefficients and codeword, Merkle tree of the folded
 //               codeword, absorb root, 24 query positions, openings in both trees    basefold.rs:483-585
 //
+// Encoding never mixes the two halves of [c || c] (chunks are at most 2^log_n long), so a codeword is two equal
+// halves, and so are the leaves of its tree: an opening stores one half (v), builds the tree over v and one node over
+// (root, root), and takes paths from the half tree.  The first fold has l = r everywhere, so it returns v whatever the
+// challenge is: v and its tree are the folded codeword and its tree (only the coefficients are folded for the final
+// value), unless a batch adds another codeword to it.  At 2^24 coefficients this leaves 2^25 node hashes of 2^26.
+//
 // XOF output block b of a root node is one compression with counter b, so the tables are
-// generated one 64-byte block per thread.  Encoding never mixes the two halves of [c || c]
-// (chunks are at most 2^log_n long), so one half is computed and written twice.  Levels below
+// generated one 64-byte block per thread.  Encoding levels below
 // 2^12 run in shared memory in one pass; higher levels go six at a time through tiles of
 // 64 consecutive values x 64 strided rows.  Each fold is fused with the first ten levels of the
 // Merkle tree over its output.  The whole opening runs without host round trips: challenges,
@@ -154,6 +159,7 @@ struct BfRound {
     const u32* prev_values; const uint4* prev_nodes;
     const u32* fold_values; const uint4* fold_nodes;
     u32 h_prev;
+    int prev_doubled;                // prev_values / prev_nodes hold one half of a codeword [v || v] (height h_prev - 1)
     u32* rec;                        // [root 4][idx 24][48 prev paths][24 folded paths]
 };
 __host__ __device__ __forceinline__ size_t bf_round_words(u32 h_prev) {
@@ -195,12 +201,20 @@ __global__ void __launch_bounds__(256) bf_round_kernel(BfRound p) {
     for (u32 item = warp; item < 3 * BF_QUERIES; item += nwarps) {
         if (item < 2 * BF_QUERIES) {
             size_t pos = idx_s[item >> 1] + ((item & 1) ? prev_half : 0);
-            mk_gather_path(p.prev_values, size_t(1) << p.h_prev, p.prev_nodes, p.h_prev, pos, out_prev + item * pw_prev, lane, 32);
+            if (p.prev_doubled) mk_gather_path_doubled(p.prev_values, p.prev_nodes, h_fold, pos, out_prev + item * pw_prev, lane, 32);
+            else mk_gather_path(p.prev_values, size_t(1) << p.h_prev, p.prev_nodes, p.h_prev, pos, out_prev + item * pw_prev, lane, 32);
         } else {
             u32 q = item - 2 * BF_QUERIES;
             mk_gather_path(p.fold_values, prev_half, p.fold_nodes, h_fold, idx_s[q], out_fold + q * pw_fold, lane, 32);
         }
     }
+}
+// The first fold of the coefficients (their values at the opened point, one coordinate per round): eval[j] = c[j] + alpha (c[j + half] - c[j]).
+// The later ones ride on the codeword folds; the first codeword fold needs no kernel.
+__global__ void __launch_bounds__(256) bf_eval_first_kernel(CoefSrc src, const u32* __restrict__ alpha, size_t half, u32* __restrict__ eval) {
+    const Fp a{*alpha};
+    for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < half; j += (size_t)gridDim.x * blockDim.x)
+        eval[j] = lerp(Fp{coef_at(src.p, src.rows, src.cols, src.log_cols_pad, j)}, Fp{coef_at(src.p, src.rows, src.cols, src.log_cols_pad, j + half)}, a).v;
 }
 // First challenge, after the commitment root has been absorbed (basefold.rs:461 / 508-513).
 __global__ void bf_begin_kernel(TrState* st, const uint4* root, const u32* point, u32 n_point, u32* alpha0, u32* rec_root) {
@@ -248,17 +262,17 @@ inline BfTables bf_tables(zkb_ctx* c, u32 log_n) {
     return tb;
 }
 
-// cw (2 * 2^log_n words) = encode of the zero-padded coefficients.
-inline void bf_encode(zkb_ctx* c, CoefSrc src, u32 log_n, const BfTables& tb, u32* cw) {
+// cw = encode of the zero-padded coefficients: 2^log_n words, the one half of the codeword, or all 2 * 2^log_n words.
+inline void bf_encode(zkb_ctx* c, CoefSrc src, u32 log_n, const BfTables& tb, u32* cw, bool both_halves) {
     const size_t n_pad = size_t(1) << log_n;
     const u32 K = log_n < (u32)BF_LOW_LOG ? log_n : (u32)BF_LOW_LOG;
-    bf_encode_low_kernel<<<(unsigned)(n_pad >> K), 256, 0, c->stream>>>(src, K, tb.t_flat, cw, n_pad, K == log_n);
+    bf_encode_low_kernel<<<(unsigned)(n_pad >> K), 256, 0, c->stream>>>(src, K, tb.t_flat, cw, n_pad, both_halves && K == log_n);
     ZKB_LAUNCHED(c);
     u32 l0 = K;
     while (l0 < log_n) {
         u32 rem = log_n - l0;
         u32 r = rem <= 6 ? rem : (rem < 12 ? (rem + 1) / 2 : 6);
-        bf_encode_high_kernel<<<(unsigned)(n_pad >> (r + 6)), 256, 0, c->stream>>>(cw, l0, r, tb.t_flat, n_pad, l0 + r == log_n);
+        bf_encode_high_kernel<<<(unsigned)(n_pad >> (r + 6)), 256, 0, c->stream>>>(cw, l0, r, tb.t_flat, n_pad, both_halves && l0 + r == log_n);
         ZKB_LAUNCHED(c);
         l0 += r;
     }
@@ -322,26 +336,27 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
     // the transcript: they run ahead on a second stream, each round into buffers of its own, while the
     // context's stream runs the hash chain (root absorb, 24 query squeezes) and the path gathers behind them.
     const bool ahead = n_point >= log_n && !c->opt_bf_in_order && !c->capturing;
-    u32* cwA = (u32*)c->scratch(2 * n_pad * 4);
-    u32* cwB = ahead ? nullptr : (u32*)c->scratch(n_pad * 4);
+    u32* cwA = (u32*)c->scratch(n_pad * 4);
+    u32* cwB = ahead ? nullptr : (u32*)c->scratch(n_pad / 2 * 4);
     u32* eval = (u32*)c->scratch((n_pad / 2 + 4) * 4);
-    uint4* treeA = (uint4*)c->scratch(mk_node_count(log_n + 1) * 16 + 16);
+    uint4* treeA = (uint4*)c->scratch(mk_node_count(log_n) * 16 + 16);
     uint4* treeB = ahead ? nullptr : (uint4*)c->scratch(mk_node_count(log_n) * 16 + 16);
     u32* alpha = (u32*)c->scratch((log_n + 1) * 4);
-    std::vector<u32*> cws;
-    std::vector<uint4*> trees;
+    std::vector<u32*> cws{cwA};            // the folded codeword of each round: the first fold's is the codeword's half itself
+    std::vector<uint4*> trees{treeA};
     if (ahead) {
-        for (u32 round = 0; round < log_n; round++) {
+        for (u32 round = 1; round < log_n; round++) {
             cws.push_back((u32*)c->scratch((size_t(4) << (log_n - round)) + 16));
             trees.push_back((uint4*)c->scratch(mk_node_count(log_n - round) * 16 + 16));
         }
     }
 
     c->prof_mark();
-    bf_encode(c, src, log_n, tb, cwA);
+    bf_encode(c, src, log_n, tb, cwA, false);
     c->prof_mark();
     MkFold none{};
-    mk_build(c, kind, MK_VALUES, cwA, 2 * n_pad, log_n + 1, treeA, none);
+    none.doubled = 1;
+    mk_build(c, kind, MK_VALUES, cwA, n_pad, log_n, treeA, none);
     c->prof_mark();
     cudaStream_t main_stream = c->stream, side = nullptr;
     if (ahead) {
@@ -351,11 +366,11 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
         ZKB_CUDA(cudaStreamWaitEvent(side, fork, 0));
     }
     pd.root_off = c->rec_alloc(4);
-    bf_begin_kernel<<<1, 1, 0, c->stream>>>(tr, treeA + mk_layer_offset(log_n + 1, log_n + 1), point_dev, n_point, alpha, c->rec_dev + pd.root_off);
+    bf_begin_kernel<<<1, 1, 0, c->stream>>>(tr, treeA + mk_node_count(log_n), point_dev, n_point, alpha, c->rec_dev + pd.root_off);
     ZKB_LAUNCHED(c);
 
-    u32* prev_cw = cwA; u32* next_cw = ahead ? cws[0] : cwB;
-    uint4* prev_tree = treeA; uint4* next_tree = ahead ? trees[0] : treeB;
+    u32* prev_cw = cwA; u32* next_cw = cwA;
+    uint4* prev_tree = treeA; uint4* next_tree = treeA;
     for (u32 round = 0; round < log_n; round++) {
         const u32 h_prev = log_n + 1 - round;
         const size_t half = size_t(1) << (h_prev - 1);
@@ -364,18 +379,23 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
         f.prev = prev_cw; f.out = next_cw;
         f.weights = tb.w_flat + ((size_t(1) << fold_level) - 1);
         f.w_len = size_t(1) << fold_level;
+        f.prev_partner = half;
         f.alpha = ahead ? point_dev + round : alpha + round;
         f.eval_src = eval; f.eval_dst = eval; f.eval_half = half / 2;
-        f.coef = src.p; f.coef_rows = src.rows; f.coef_cols = src.cols; f.coef_log_cols_pad = src.log_cols_pad;
-        f.eval_from_coef = round == 0;
+        auto fold = [&] {
+            if (round == 0) {
+                bf_eval_first_kernel<<<grid_for(c, half / 2), 256, 0, c->stream>>>(src, f.alpha, half / 2, eval);
+                ZKB_LAUNCHED(c);
+            } else mk_build(c, kind, MK_FOLD, nullptr, half, h_prev - 1, next_tree, f);
+        };
         if (ahead) {
             c->stream = side;
-            try { mk_build(c, kind, MK_FOLD, nullptr, half, h_prev - 1, next_tree, f); } catch (...) { c->stream = main_stream; throw; }
+            try { fold(); } catch (...) { c->stream = main_stream; throw; }
             c->stream = main_stream;
             ZKB_CUDA(cudaEventRecord(c->side_event(round), side));
             ZKB_CUDA(cudaStreamWaitEvent(main_stream, c->side_event(round), 0));
         } else {
-            mk_build(c, kind, MK_FOLD, nullptr, half, h_prev - 1, next_tree, f);
+            fold();
         }
         c->prof_mark();
         BfRound rp{};
@@ -383,6 +403,7 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
         rp.alpha_next = round + 1 < log_n ? alpha + round + 1 : nullptr;
         rp.prev_values = prev_cw; rp.prev_nodes = prev_tree; rp.fold_values = next_cw; rp.fold_nodes = next_tree;
         rp.h_prev = h_prev;
+        rp.prev_doubled = round == 0;
         size_t off = c->rec_alloc(bf_round_words(h_prev));
         rp.rec = c->rec_dev + off;
         pd.round_off.push_back(off);
@@ -392,6 +413,8 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
         if (ahead) {
             prev_cw = next_cw; prev_tree = next_tree;
             if (round + 1 < log_n) { next_cw = cws[round + 1]; next_tree = trees[round + 1]; }
+        } else if (round == 0) {
+            next_cw = cwB; next_tree = treeB;
         } else {
             std::swap(prev_cw, next_cw);
             std::swap(prev_tree, next_tree);

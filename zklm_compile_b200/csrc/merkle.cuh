@@ -118,11 +118,13 @@ struct MkFold {
     u32* eval_src;        // coefficient buffer being evaluated (eval_half * 2 live values), or null
     u32* eval_dst;        // where the folded coefficients go (may equal eval_src)
     size_t w_len, eval_half;
-    // first round only: coefficients are read through a row-padded view of a matrix
-    const u32* coef; u32 coef_rows, coef_cols, coef_log_cols_pad; int eval_from_coef;
     // batch openings: values added to the folded codeword before it is stored and hashed (the already scaled sum of the
     // codewords that join the chain at this length), or null
-    const u32* add;
+    const u32* add; size_t add_mask;      // add[j & add_mask]: a joining codeword is [v || v], only v is summed
+    // prev[j + prev_partner] is the other value of a pair: half of the codeword's length, or 0 while the codeword is
+    // [c || c] and only c is stored (its two values are then the same, and the fold leaves c as it is)
+    size_t prev_partner;
+    int doubled;          // the launch that reaches the root also stores the node over (root, root) behind it: the root of [c || c]
 };
 
 __device__ __forceinline__ u32 coef_at(const u32* __restrict__ p, u32 rows, u32 cols, u32 log_cols_pad, size_t i) {
@@ -154,25 +156,18 @@ __global__ void __launch_bounds__(MK_THREADS) mk_tile_kernel(const u32* __restri
             bufA[i] = make_uint4(g < n_valid ? values[g] : 0u, 0, 0, 0);
         }
     } else {
-        const size_t half = n_in;
         const Fp alpha{*fold.alpha};
         const Fp two_inv{1073741824u};
         for (size_t i = threadIdx.x; i < tile; i += MK_THREADS) {
             size_t j = base + i;
-            Fp l{fold.prev[j]}, r{fold.prev[j + half]};
+            Fp l{fold.prev[j]}, r{fold.prev[j + fold.prev_partner]};
             Fp w{fold.weights[j & (fold.w_len - 1)]};
             Fp f = (l + r) * two_inv + alpha * ((l - r) * w);
-            if (fold.add) f = f + Fp{fold.add[j]};
+            if (fold.add) f = f + Fp{fold.add[j & fold.add_mask]};
             fold.out[j] = f.v;
             bufA[i] = make_uint4(f.v, 0, 0, 0);
             if (fold.eval_dst && j < fold.eval_half) {
-                Fp a, b;
-                if (fold.eval_from_coef) {
-                    a.v = coef_at(fold.coef, fold.coef_rows, fold.coef_cols, fold.coef_log_cols_pad, j);
-                    b.v = coef_at(fold.coef, fold.coef_rows, fold.coef_cols, fold.coef_log_cols_pad, j + fold.eval_half);
-                } else {
-                    a.v = fold.eval_src[j]; b.v = fold.eval_src[j + fold.eval_half];
-                }
+                const Fp a{fold.eval_src[j]}, b{fold.eval_src[j + fold.eval_half]};
                 fold.eval_dst[j] = ((fp_one() - alpha) * a + alpha * b).v;
             }
         }
@@ -196,6 +191,8 @@ __global__ void __launch_bounds__(MK_THREADS) mk_tile_kernel(const u32* __restri
         uint4* t = cur; cur = nxt; nxt = t;
         cnt = out_cnt;
     }
+    if (fold.doubled && k == h && threadIdx.x == 0)
+        nodes[mk_node_count(h)] = KIND == NODE_AES_MMO ? aes_node(cur[0], cur[0], t0_s, sb_s) : b3_node(cur[0], cur[0]);
 }
 
 // Raw authentication data of opened positions: for position p of a tree of height h over
@@ -215,6 +212,18 @@ __device__ inline void mk_gather_path(const u32* __restrict__ values, size_t n_v
             u32* o = out + 2 + 4 * (size_t)(k - 2);
             o[0] = d.x; o[1] = d.y; o[2] = d.z; o[3] = d.w;
         }
+    }
+}
+// The same path out of the tree of height h + 1 over [v || v], of which the tree of height h over v is stored: below the
+// root both halves have the same nodes, and the last sibling is the other half's root, which is the stored one.
+__device__ inline void mk_gather_path_doubled(const u32* __restrict__ values, const uint4* __restrict__ nodes, u32 h, size_t p, u32* out,
+                                              int lane, int nlanes) {
+    const size_t n = size_t(1) << h;
+    mk_gather_path(values, n, nodes, h, p & (n - 1), out, lane, nlanes);
+    if (lane == 0) {
+        const uint4 d = nodes[mk_layer_offset(h, h)];
+        u32* o = out + 2 + 4 * (size_t)(h - 1);
+        o[0] = d.x; o[1] = d.y; o[2] = d.z; o[3] = d.w;
     }
 }
 // Positions given by the host (the stand-alone Merkle entry points).
