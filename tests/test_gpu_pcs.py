@@ -33,6 +33,26 @@ def test_merkle_root_and_layers(ctx, kind, n):
 
 
 @pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("n", [(1 << 19) + 1, (1 << 20) + 1, 1 << 21])
+def test_merkle_tree_whose_levels_are_built_a_subtree_per_thread(ctx, kind, n):
+    """From 2^20 inputs to a level on: the first and last threads' subtrees, the ragged end, and positions spread over the CTAs."""
+    v = rnd(n, n)
+    top = 1 << (n - 1).bit_length()
+    idx = sorted({0, 1, 15, 16, 4095, 4096, n - 1, min(n, top - 1), top - 1} | set(range(0, top, top // 61)))
+    assert zp.merkle_root(ctx, v, kind) == O.merkle_root(v, kind)
+    assert zp.merkle_batch_open(ctx, v, idx, kind) == O.merkle_batch_open(v, kind, idx)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("n", [(1 << 20) + 3, 1 << 21])
+def test_basefold_with_folds_of_a_subtree_per_thread(ctx, kind, n):
+    c, pt = rnd(400 + n, n), rnd(500 + n, (n - 1).bit_length())
+    tg, to = zk.Transcript(ctx, b"bf-lane"), O.Transcript(b"bf-lane")
+    assert zp.basefold_commit_and_prove(ctx, tg, c, pt, kind) == O.basefold_commit_and_prove(to, c, pt, kind)
+    assert tg.squeeze() == to.squeeze()
+
+
+@pytest.mark.parametrize("kind", KINDS)
 def test_merkle_batch_open_bytes(ctx, kind):
     v = rnd(7, 3000)
     for idx in ([3, 3, 2, 2999, 4095, 2048, 0, 1], [17], list(range(40)), [4095, 0]):

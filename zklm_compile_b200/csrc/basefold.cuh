@@ -280,6 +280,14 @@ inline void bf_encode(zkb_ctx* c, CoefSrc src, u32 log_n, const BfTables& tb, u3
 
 template <int KIND>
 inline void mk_launch(zkb_ctx* c, int mode, const u32* values, size_t n_valid, size_t n_in, u32 k0, u32 h, uint4* nodes, const MkFold& f) {
+    if (n_in >= MK_LANE_MIN) {
+        const unsigned grid = (unsigned)(n_in / (MK_LANE_THREADS * MK_LANE));
+        if (mode == MK_VALUES) mk_lane_kernel<KIND, MK_VALUES><<<grid, MK_LANE_THREADS, mk_lane_smem(KIND), c->stream>>>(values, n_valid, k0, h, nodes, f);
+        else if (mode == MK_DIGESTS) mk_lane_kernel<KIND, MK_DIGESTS><<<grid, MK_LANE_THREADS, mk_lane_smem(KIND), c->stream>>>(values, n_valid, k0, h, nodes, f);
+        else mk_lane_kernel<KIND, MK_FOLD><<<grid, MK_LANE_THREADS, mk_lane_smem(KIND), c->stream>>>(values, n_valid, k0, h, nodes, f);
+        ZKB_LAUNCHED(c);
+        return;
+    }
     const size_t tile = n_in < (size_t)MK_TILE ? n_in : (size_t)MK_TILE;
     const unsigned grid = (unsigned)(n_in / tile);
     if (mode == MK_VALUES) mk_tile_kernel<KIND, MK_VALUES><<<grid, MK_THREADS, 0, c->stream>>>(values, n_valid, n_in, k0, h, nodes, f);
@@ -295,7 +303,8 @@ inline void mk_build(zkb_ctx* c, int kind, int first_mode, const u32* values, si
         size_t n_in = size_t(1) << (h - k0);
         if (kind == NODE_AES_MMO) mk_launch<NODE_AES_MMO>(c, mode, values, n_valid, n_in, k0, h, nodes, f);
         else mk_launch<NODE_BLAKE3>(c, mode, values, n_valid, n_in, k0, h, nodes, f);
-        k0 += (h - k0) < (u32)MK_TILE_LOG ? (h - k0) : (u32)MK_TILE_LOG;
+        const u32 levels = n_in >= MK_LANE_MIN ? (u32)MK_LANE_LOG : (u32)MK_TILE_LOG;
+        k0 += (h - k0) < levels ? (h - k0) : levels;
         mode = MK_DIGESTS;
     }
 }
@@ -309,6 +318,9 @@ inline void aes_tables_upload() {
     AesTables t = aes_make_tables();
     ZKB_CUDA(cudaMemcpyToSymbol(AES_T0, t.t0, sizeof(t.t0)));
     ZKB_CUDA(cudaMemcpyToSymbol(AES_SBOX, t.sbox, sizeof(t.sbox)));
+    // table and staged leaves together exceed the 48 KB that need no opt-in
+    ZKB_CUDA(cudaFuncSetAttribute(mk_lane_kernel<NODE_AES_MMO, MK_VALUES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mk_lane_smem(NODE_AES_MMO)));
+    ZKB_CUDA(cudaFuncSetAttribute(mk_lane_kernel<NODE_AES_MMO, MK_FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mk_lane_smem(NODE_AES_MMO)));
     done[dev] = true;
 }
 

@@ -9,7 +9,8 @@
 // A tree of height h over 2^h leaves stores layers 1..h (layer k has 2^(h-k) nodes) back to
 // back: layer k starts at node offset 2^h - 2^(h-k+1); the root is node 2^h - 2.  One launch
 // of mk_tile_kernel builds up to MK_TILE_LOG levels: each CTA owns MK_TILE consecutive inputs,
-// keeps the running level in shared memory and writes every level it produces.  A 32-byte node
+// keeps the running level in shared memory and writes every level it produces; levels of 2^20 inputs
+// and more go to mk_lane_kernel, four at a time.  A 32-byte node
 // input is a single blake3 block, so one node costs one compression; the kernel is bound by
 // integer issue, not by bandwidth (16 bytes read and 8 written per compression on average).
 #pragma once
@@ -21,9 +22,11 @@ enum NodeHash : int { NODE_BLAKE3 = 0, NODE_AES_MMO = 1 };
 
 // ---- blake3 node: one block of 32 bytes, flags CHUNK_START | CHUNK_END | ROOT -------------------
 // Message words 8..15 are zero, so with the schedule resolved at compile time half of the
-// message additions disappear.
+// message additions disappear; over two leaves (LEAVES) only words 0 and 4 are not zero.
+template <bool LEAVES = false>
 __device__ __forceinline__ uint4 b3_node(uint4 l, uint4 r) {
     u32 w[16] = {l.x, l.y, l.z, l.w, r.x, r.y, r.z, r.w, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (LEAVES) w[1] = w[2] = w[3] = w[5] = w[6] = w[7] = 0;
     u32 s0 = 0x6a09e667u, s1 = 0xbb67ae85u, s2 = 0x3c6ef372u, s3 = 0xa54ff53au;
     u32 s4 = 0x510e527fu, s5 = 0x9b05688cu, s6 = 0x1f83d9abu, s7 = 0x5be0cd19u;
     u32 s8 = 0x6a09e667u, s9 = 0xbb67ae85u, s10 = 0x3c6ef372u, s11 = 0xa54ff53au;
@@ -95,6 +98,47 @@ __device__ __forceinline__ uint4 aes_node(uint4 l, uint4 r, const u32* __restric
     return make_uint4(c0 ^ x0, c1 ^ x1, c2 ^ x2, c3 ^ x3);
 }
 
+// The same node with T0 replicated once per bank, so that the lookups of a warp never meet in one: word x * 32 + b
+// of `rep` is T0[x], lane b reads column b.  With one copy a lookup takes the warp three to four passes.  The
+// last round's S[x] is the second byte of T0[x].
+constexpr int AES_REP_WORDS = 256 * 32;
+__device__ __forceinline__ void aes_rep_fill(u32* rep) {
+    for (u32 i = threadIdx.x; i < (u32)AES_REP_WORDS; i += blockDim.x) rep[i] = AES_T0[i >> 5];
+}
+template <int BYTE>
+__device__ __forceinline__ u32 aes_rep_at(const u32* __restrict__ rep, u32 lane4, u32 c) {
+    const u32 sh = BYTE == 0 ? c << 7 : c >> (8 * BYTE - 7);
+    return *reinterpret_cast<const u32*>(reinterpret_cast<const unsigned char*>(rep) + ((sh & 0x7f80u) | lane4));
+}
+__device__ __forceinline__ u32 aes_rep_column(const u32* __restrict__ rep, u32 l4, u32 a, u32 b, u32 c, u32 d) {
+    return aes_rep_at<0>(rep, l4, a) ^ rotl8(aes_rep_at<1>(rep, l4, b), 1) ^ rotl8(aes_rep_at<2>(rep, l4, c), 2) ^ rotl8(aes_rep_at<3>(rep, l4, d), 3);
+}
+__device__ __forceinline__ u32 aes_rep_last(const u32* __restrict__ rep, u32 l4, u32 a, u32 b, u32 c, u32 d) {
+    const u32 lo = __byte_perm(aes_rep_at<0>(rep, l4, a), aes_rep_at<1>(rep, l4, b), 0x0051);
+    const u32 hi = __byte_perm(aes_rep_at<2>(rep, l4, c), aes_rep_at<3>(rep, l4, d), 0x0051);
+    return __byte_perm(lo, hi, 0x5410);
+}
+__device__ __forceinline__ uint4 aes_node_rep(uint4 l, uint4 r, const u32* __restrict__ rep) {
+    const u32 l4 = (threadIdx.x & 31) * 4;
+    const u32 x0 = l.x ^ r.x, x1 = l.y ^ r.y, x2 = l.z ^ r.z, x3 = l.w ^ r.w;
+    u32 c0 = x0, c1 = x1, c2 = x2, c3 = x3;
+#pragma unroll
+    for (int rd = 0; rd < 10; rd++) {
+        const uint4 k = (rd & 1) ? r : l;
+        c0 ^= k.x; c1 ^= k.y; c2 ^= k.z; c3 ^= k.w;
+        u32 n0, n1, n2, n3;
+        if (rd < 9) {
+            n0 = aes_rep_column(rep, l4, c0, c1, c2, c3); n1 = aes_rep_column(rep, l4, c1, c2, c3, c0);
+            n2 = aes_rep_column(rep, l4, c2, c3, c0, c1); n3 = aes_rep_column(rep, l4, c3, c0, c1, c2);
+        } else {
+            n0 = aes_rep_last(rep, l4, c0, c1, c2, c3); n1 = aes_rep_last(rep, l4, c1, c2, c3, c0);
+            n2 = aes_rep_last(rep, l4, c2, c3, c0, c1); n3 = aes_rep_last(rep, l4, c3, c0, c1, c2);
+        }
+        c0 = n0; c1 = n1; c2 = n2; c3 = n3;
+    }
+    return make_uint4(c0 ^ x0, c1 ^ x1, c2 ^ x2, c3 ^ x3);
+}
+
 // ---- tree storage ---------------------------------------------------------------------------------
 __host__ __device__ __forceinline__ size_t mk_layer_offset(u32 h, u32 k) { return (size_t(1) << h) - (size_t(1) << (h - k + 1)); }
 __host__ __device__ __forceinline__ size_t mk_node_count(u32 h) { return (size_t(1) << h) - 1; }
@@ -132,6 +176,21 @@ __device__ __forceinline__ u32 coef_at(const u32* __restrict__ p, u32 rows, u32 
     return (r < rows && c < cols) ? p[r * cols + c] : 0u;
 }
 
+// One value of the folded codeword (and, below eval_half, of the folded coefficients).
+__device__ __forceinline__ u32 mk_fold_value(const MkFold& fold, Fp alpha, size_t j) {
+    const Fp two_inv{1073741824u};
+    Fp l{fold.prev[j]}, r{fold.prev[j + fold.prev_partner]};
+    Fp w{fold.weights[j & (fold.w_len - 1)]};
+    Fp f = (l + r) * two_inv + alpha * ((l - r) * w);
+    if (fold.add) f = f + Fp{fold.add[j & fold.add_mask]};
+    fold.out[j] = f.v;
+    if (fold.eval_dst && j < fold.eval_half) {
+        const Fp a{fold.eval_src[j]}, b{fold.eval_src[j + fold.eval_half]};
+        fold.eval_dst[j] = ((fp_one() - alpha) * a + alpha * b).v;
+    }
+    return f.v;
+}
+
 // One CTA: MK_TILE inputs (fewer when the whole level is smaller) -> up to MK_TILE_LOG layers.
 // n_in = number of inputs at level k0 (a power of two); h = height of the tree.
 template <int KIND, int MODE>
@@ -157,20 +216,7 @@ __global__ void __launch_bounds__(MK_THREADS) mk_tile_kernel(const u32* __restri
         }
     } else {
         const Fp alpha{*fold.alpha};
-        const Fp two_inv{1073741824u};
-        for (size_t i = threadIdx.x; i < tile; i += MK_THREADS) {
-            size_t j = base + i;
-            Fp l{fold.prev[j]}, r{fold.prev[j + fold.prev_partner]};
-            Fp w{fold.weights[j & (fold.w_len - 1)]};
-            Fp f = (l + r) * two_inv + alpha * ((l - r) * w);
-            if (fold.add) f = f + Fp{fold.add[j & fold.add_mask]};
-            fold.out[j] = f.v;
-            bufA[i] = make_uint4(f.v, 0, 0, 0);
-            if (fold.eval_dst && j < fold.eval_half) {
-                const Fp a{fold.eval_src[j]}, b{fold.eval_src[j + fold.eval_half]};
-                fold.eval_dst[j] = ((fp_one() - alpha) * a + alpha * b).v;
-            }
-        }
+        for (size_t i = threadIdx.x; i < tile; i += MK_THREADS) bufA[i] = make_uint4(mk_fold_value(fold, alpha, base + i), 0, 0, 0);
     }
     __syncthreads();
 
@@ -193,6 +239,58 @@ __global__ void __launch_bounds__(MK_THREADS) mk_tile_kernel(const u32* __restri
     }
     if (fold.doubled && k == h && threadIdx.x == 0)
         nodes[mk_node_count(h)] = KIND == NODE_AES_MMO ? aes_node(cur[0], cur[0], t0_s, sb_s) : b3_node(cur[0], cur[0]);
+}
+
+// Four levels of a level that is large enough to give every thread a subtree of its own: 16 consecutive inputs, their
+// fifteen nodes one after the other in post-order, the nodes that wait for their sibling in registers.  No lane is ever
+// idle and no barrier separates the levels; in a tile the last five levels run on part of a warp, and most warps wait.
+// Leaves are staged (and folded) through shared memory with coalesced accesses, one word of padding per thread.
+constexpr int MK_LANE_LOG = 4, MK_LANE = 1 << MK_LANE_LOG, MK_LANE_THREADS = 256;
+constexpr size_t mk_lane_smem(int kind) { return kind == NODE_AES_MMO ? AES_REP_WORDS * 4 : 0; }
+constexpr size_t MK_LANE_MIN = size_t(1) << 20;      // inputs: below, the subtrees are too few to fill the GPU
+template <int KIND, int MODE>
+__global__ void __launch_bounds__(MK_LANE_THREADS) mk_lane_kernel(const u32* __restrict__ values, size_t n_valid, u32 k0, u32 h,
+                                                                 uint4* __restrict__ nodes, MkFold fold) {
+    __shared__ u32 leaf[MODE == MK_DIGESTS ? 1 : MK_LANE_THREADS * (MK_LANE + 1)];
+    extern __shared__ __align__(16) u32 rep[];               // AES: the replicated table (mk_lane_smem bytes)
+    if (KIND == NODE_AES_MMO) aes_rep_fill(rep);
+    const size_t base = (size_t)blockIdx.x * (MK_LANE_THREADS * MK_LANE);
+    if (MODE != MK_DIGESTS) {
+        Fp alpha{0};
+        if (MODE == MK_FOLD) alpha.v = *fold.alpha;
+        for (u32 e = threadIdx.x; e < MK_LANE_THREADS * MK_LANE; e += MK_LANE_THREADS) {
+            const size_t g = base + e;
+            u32 v;
+            if (MODE == MK_FOLD) v = mk_fold_value(fold, alpha, g);
+            else v = g < n_valid ? values[g] : 0u;
+            leaf[e + (e >> MK_LANE_LOG)] = v;
+        }
+    }
+    __syncthreads();
+    const size_t t = base / MK_LANE + threadIdx.x;          // this thread's node four levels up
+    const u32* mine = leaf + threadIdx.x * (MK_LANE + 1);
+    const uint4* in = MODE == MK_DIGESTS ? nodes + mk_layer_offset(h, k0) + t * MK_LANE : nullptr;
+    uint4 w1 = make_uint4(0, 0, 0, 0), w2 = w1, w3 = w1, d = w1;       // waiting nodes of levels 1..3
+    u32 pair = 0, lvl = 0;
+    while (lvl < MK_LANE_LOG) {                              // the same for all threads
+        if (MODE != MK_DIGESTS && lvl == 0) {
+            const uint4 l = make_uint4(mine[2 * pair], 0, 0, 0), r = make_uint4(mine[2 * pair + 1], 0, 0, 0);
+            d = KIND == NODE_AES_MMO ? aes_node_rep(l, r, rep) : b3_node<true>(l, r);
+        } else {
+            uint4 l, r = d;
+            if (lvl == 0) { l = in[2 * pair]; r = in[2 * pair + 1]; }
+            else l = lvl == 1 ? w1 : (lvl == 2 ? w2 : w3);
+            d = KIND == NODE_AES_MMO ? aes_node_rep(l, r, rep) : b3_node(l, r);
+        }
+        const u32 q = pair >> lvl;                           // index of the node within this thread's nodes of its level
+        lvl++;
+        nodes[mk_layer_offset(h, k0 + lvl) + (t << (MK_LANE_LOG - lvl)) + q] = d;
+        if (lvl < MK_LANE_LOG && !(q & 1)) {                 // a left child waits; the next pair of inputs follows
+            if (lvl == 1) w1 = d; else if (lvl == 2) w2 = d; else w3 = d;
+            lvl = 0;
+            pair++;
+        }
+    }
 }
 
 // Raw authentication data of opened positions: for position p of a tree of height h over
