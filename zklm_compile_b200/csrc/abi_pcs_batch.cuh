@@ -156,6 +156,8 @@ BfbPending bfb_enqueue(zkb_bf_batch* B, TrState* tr, bool individual) {
     u32* prev_cw = cw0;
     uint4* prev_tree = tree0;
     size_t next_group = 1;
+    BfRounds rounds{};
+    rounds.tr = tr; rounds.point = fold_point; rounds.n_point = log_n;
     for (u32 round = 0; round < log_n; round++) {
         const u32 h_prev = log_n + 1 - round;
         const size_t half = size_t(1) << (h_prev - 1);           // length of the folded codeword
@@ -190,12 +192,8 @@ BfbPending bfb_enqueue(zkb_bf_batch* B, TrState* tr, bool individual) {
             }
             if (!reuse) mk_build(c, kind, MK_FOLD, nullptr, half, h_prev - 1, next_tree, f);
             c->stream = main_stream;
-            if (!in_order) {
-                ZKB_CUDA(cudaEventRecord(c->side_event(round), work));
-                ZKB_CUDA(cudaStreamWaitEvent(main_stream, c->side_event(round), 0));
-            }
-            BfRound rp{};
-            rp.tr = tr; rp.point = fold_point; rp.n_point = log_n; rp.round = round; rp.log_n = log_n;
+            if (!in_order) ZKB_CUDA(cudaEventRecord(c->side_event(round), work));
+            BfRound& rp = rounds.r[round];
             rp.alpha_next = round + 1 < log_n ? fold_point + log_n : nullptr;    // the value is already in fold_point; the slot behind it takes the copy
             rp.prev_values = prev_cw; rp.prev_nodes = prev_tree; rp.fold_values = next_cw; rp.fold_nodes = next_tree;
             rp.h_prev = h_prev;
@@ -203,18 +201,24 @@ BfbPending bfb_enqueue(zkb_bf_batch* B, TrState* tr, bool individual) {
             const size_t off = c->rec_alloc(bf_round_words(h_prev));
             rp.rec = c->rec_dev + off;
             pd.round_off.push_back(off);
-            bf_round_kernel<<<1, 256, exclusive_smem(bf_round_kernel, c), c->stream>>>(rp);
-            ZKB_LAUNCHED(c);
-            // the joined polynomials' own trees, opened at this round's positions (:1330-1345)
-            for (u32 i = first; i < first + count; i++) {
-                const u32 h = B->e[i].log_n + 1;
-                const size_t o = c->rec_alloc(2 * (size_t)BF_QUERIES * (2 + 4 * (size_t)(h - 1)));
-                bfb_open_kernel<<<1, 256, 0, c->stream>>>(B->e[i].cw, B->e[i].tree, h, c->rec_dev + off + 4, u32(1) << B->e[i].log_n, c->rec_dev + o);
-                ZKB_LAUNCHED(c);
-                pd.add_opens.push_back(BfbPending::Open{round, i, o});
-            }
+            // the joined polynomials' own trees are opened at this round's positions (:1330-1345)
+            for (u32 i = first; i < first + count; i++)
+                pd.add_opens.push_back(BfbPending::Open{round, i, c->rec_alloc(2 * (size_t)BF_QUERIES * (2 + 4 * (size_t)B->e[i].log_n))});
         } catch (...) { c->stream = main_stream; throw; }
         prev_cw = next_cw; prev_tree = next_tree;
+    }
+    // every round has buffers of its own, so the chain runs through and the paths of all rounds are gathered behind it
+    for (rounds.first = 0; rounds.first < log_n; rounds.first += rounds.count) {
+        rounds.count = in_order ? log_n : bf_chain_rounds(rounds.first, log_n);
+        if (!in_order) ZKB_CUDA(cudaStreamWaitEvent(main_stream, c->side_event(rounds.first + rounds.count - 1), 0));
+        bf_launch_chain(c, rounds);
+    }
+    rounds.first = 0; rounds.count = log_n;
+    bf_launch_gather(c, rounds);
+    for (const BfbPending::Open& o : pd.add_opens) {
+        const zkb_bf_batch::Entry& e = B->e[o.poly];
+        bfb_open_kernel<<<1, 256, 0, c->stream>>>(e.cw, e.tree, e.log_n + 1, c->rec_dev + pd.round_off[o.round] + 4, u32(1) << e.log_n, c->rec_dev + o.off);
+        ZKB_LAUNCHED(c);
     }
     pd.final_idx_off = c->rec_alloc(BF_QUERIES);
     bfb_final_kernel<<<1, 1, 0, c->stream>>>(tr, (u32(1) << log_n) - 1, c->rec_dev + pd.final_idx_off);

@@ -151,16 +151,21 @@ __global__ void __launch_bounds__(256) bf_encode_high_kernel(u32* __restrict__ c
 // ---- per-round transcript step and openings ------------------------------------------------------
 constexpr u32 BF_QUERIES = 24;       // pcs.rs:19
 struct BfRound {
-    TrState* tr;
-    const u32* point; u32 n_point;   // device-resident evaluation point
-    u32 round, log_n;
-    u32* alpha_next;                 // where the next round's challenge goes (null after the last round)
     // trees: prev has height h_prev over prev_values, folded has height h_prev - 1
     const u32* prev_values; const uint4* prev_nodes;
     const u32* fold_values; const uint4* fold_nodes;
     u32 h_prev;
     int prev_doubled;                // prev_values / prev_nodes hold one half of a codeword [v || v] (height h_prev - 1)
+    u32* alpha_next;                 // where the next round's challenge goes (null after the last round)
     u32* rec;                        // [root 4][idx 24][48 prev paths][24 folded paths]
+};
+// The rounds [first, first + count) of an opening.
+constexpr u32 BF_MAX_ROUNDS = 28;
+struct BfRounds {
+    TrState* tr;
+    const u32* point; u32 n_point;   // device-resident evaluation point
+    u32 first, count;
+    BfRound r[BF_MAX_ROUNDS];
 };
 __host__ __device__ __forceinline__ size_t bf_round_words(u32 h_prev) {
     size_t pw_prev = 2 + 4 * (size_t)(h_prev - 1), pw_fold = h_prev >= 2 ? 2 + 4 * (size_t)(h_prev - 2) : 2;
@@ -172,41 +177,44 @@ __device__ __forceinline__ u32 bf_next_alpha(Tr& tr, const u32* point, u32 n_poi
     if (round < n_point) { u32 a = point[round]; tr_absorb_u32(tr, a); return a; }
     return tr_squeeze(tr);
 }
-__global__ void __launch_bounds__(256) bf_round_kernel(BfRound p) {
+// The transcript's part of some rounds: absorb the folded root, squeeze the query positions, take the next challenge.  This
+// is the opening's critical path, so nothing else is in it: the paths are gathered by bf_gather_kernel, off the chain.
+__global__ void __launch_bounds__(32) bf_chain_kernel(const __grid_constant__ BfRounds a) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
-    __shared__ u32 idx_s[BF_QUERIES];
-    const u32 h_fold = p.h_prev - 1;
-    const uint4 root = p.fold_nodes[mk_layer_offset(h_fold, h_fold)];
-    if (threadIdx.x == 0) {
-        Tr tr;
-        tr_load(tr, p.tr, trbuf);
+    if (threadIdx.x) return;
+    Tr tr;
+    tr_load(tr, a.tr, trbuf);
+    for (u32 round = a.first; round < a.first + a.count; round++) {
+        const BfRound& p = a.r[round];
+        const u32 h_fold = p.h_prev - 1;
+        const uint4 root = p.fold_nodes[mk_layer_offset(h_fold, h_fold)];
         u32 rw[4] = {root.x, root.y, root.z, root.w};
         tr_absorb_words<4>(tr, rw);
         p.rec[0] = root.x; p.rec[1] = root.y; p.rec[2] = root.z; p.rec[3] = root.w;
         const u32 prev_half_mask = (1u << (p.h_prev - 1)) - 1;
-        for (u32 q = 0; q < BF_QUERIES; q++) {
-            u32 v = tr_squeeze(tr) & prev_half_mask;     // (squeeze mod 2^h_prev) mod prev_half
-            idx_s[q] = v;
-            p.rec[4 + q] = v;
-        }
-        if (p.alpha_next) *p.alpha_next = bf_next_alpha(tr, p.point, p.n_point, p.round + 1);
-        tr_store(tr, p.tr);
+        for (u32 q = 0; q < BF_QUERIES; q++) p.rec[4 + q] = tr_squeeze(tr) & prev_half_mask;     // (squeeze mod 2^h_prev) mod prev_half
+        if (p.alpha_next) *p.alpha_next = bf_next_alpha(tr, a.point, a.n_point, round + 1);
     }
-    __syncthreads();
+    tr_store(tr, a.tr);
+}
+// The opened paths of those rounds, one warp each: blockIdx.y is the round, 3 * BF_QUERIES paths to a round.
+constexpr u32 BF_GATHER_WARPS = 8;
+__global__ void __launch_bounds__(32 * BF_GATHER_WARPS) bf_gather_kernel(const __grid_constant__ BfRounds a) {
+    const BfRound& p = a.r[a.first + blockIdx.y];
+    const u32 h_fold = p.h_prev - 1;
+    const u32* idx = p.rec + 4;
     const size_t prev_half = size_t(1) << (p.h_prev - 1);
     const size_t pw_prev = 2 + 4 * (size_t)(p.h_prev - 1), pw_fold = h_fold >= 1 ? 2 + 4 * (size_t)(h_fold - 1) : 2;
     u32* out_prev = p.rec + 4 + BF_QUERIES;
     u32* out_fold = out_prev + 2 * BF_QUERIES * pw_prev;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    for (u32 item = warp; item < 3 * BF_QUERIES; item += nwarps) {
-        if (item < 2 * BF_QUERIES) {
-            size_t pos = idx_s[item >> 1] + ((item & 1) ? prev_half : 0);
-            if (p.prev_doubled) mk_gather_path_doubled(p.prev_values, p.prev_nodes, h_fold, pos, out_prev + item * pw_prev, lane, 32);
-            else mk_gather_path(p.prev_values, size_t(1) << p.h_prev, p.prev_nodes, p.h_prev, pos, out_prev + item * pw_prev, lane, 32);
-        } else {
-            u32 q = item - 2 * BF_QUERIES;
-            mk_gather_path(p.fold_values, prev_half, p.fold_nodes, h_fold, idx_s[q], out_fold + q * pw_fold, lane, 32);
-        }
+    const u32 lane = threadIdx.x & 31, item = blockIdx.x * BF_GATHER_WARPS + (threadIdx.x >> 5);
+    if (item < 2 * BF_QUERIES) {
+        const size_t pos = idx[item >> 1] + ((item & 1) ? prev_half : 0);
+        if (p.prev_doubled) mk_gather_path_doubled(p.prev_values, p.prev_nodes, h_fold, pos, out_prev + item * pw_prev, lane, 32);
+        else mk_gather_path(p.prev_values, size_t(1) << p.h_prev, p.prev_nodes, p.h_prev, pos, out_prev + item * pw_prev, lane, 32);
+    } else if (item < 3 * BF_QUERIES) {
+        const u32 q = item - 2 * BF_QUERIES;
+        mk_gather_path(p.fold_values, prev_half, p.fold_nodes, h_fold, idx[q], out_fold + q * pw_fold, lane, 32);
     }
 }
 // The first fold of the coefficients (their values at the opened point, one coordinate per round): eval[j] = c[j] + alpha (c[j + half] - c[j]).
@@ -332,6 +340,24 @@ struct BfPending {
     std::vector<size_t> round_off;
 };
 
+inline void bf_launch_gather(zkb_ctx* c, const BfRounds& a) {
+    bf_gather_kernel<<<dim3((3 * BF_QUERIES + BF_GATHER_WARPS - 1) / BF_GATHER_WARPS, a.count), 32 * BF_GATHER_WARPS, 0, c->stream>>>(a);
+    ZKB_LAUNCHED(c);
+}
+inline void bf_launch_chain(zkb_ctx* c, const BfRounds& a) {
+    bf_chain_kernel<<<1, 32, exclusive_smem(bf_chain_kernel, c), c->stream>>>(a);
+    ZKB_LAUNCHED(c);
+}
+// How many rounds the chain launch that starts at `round` takes when the trees run ahead on another stream: one while the
+// folded codewords are long (the next tree is still being built when this round's positions are known), then four,
+// then all the rest, whose small trees are finished long before the chain gets to them (58 us a round at the slowest,
+// about 13 us a tree).
+inline u32 bf_chain_rounds(u32 round, u32 log_n) {
+    const u32 long_rounds = log_n > 18 ? log_n - 18 : 0;
+    const u32 n = round < long_rounds ? 1 : (round == long_rounds ? 4 : log_n);
+    return n < log_n - round ? n : log_n - round;
+}
+
 // Enqueue commit + opening of the polynomial `src` (num_coeffs live coefficients, padded view of
 // 2^log_n) at the device-resident point.  The transcript first absorbs the commitment root.
 inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t num_coeffs, u32 log_n, const u32* point_dev, u32 n_point,
@@ -383,6 +409,8 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
 
     u32* prev_cw = cwA; u32* next_cw = cwA;
     uint4* prev_tree = treeA; uint4* next_tree = treeA;
+    BfRounds rounds{};
+    rounds.tr = tr; rounds.point = point_dev; rounds.n_point = n_point;
     for (u32 round = 0; round < log_n; round++) {
         const u32 h_prev = log_n + 1 - round;
         const size_t half = size_t(1) << (h_prev - 1);
@@ -405,13 +433,11 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
             try { fold(); } catch (...) { c->stream = main_stream; throw; }
             c->stream = main_stream;
             ZKB_CUDA(cudaEventRecord(c->side_event(round), side));
-            ZKB_CUDA(cudaStreamWaitEvent(main_stream, c->side_event(round), 0));
         } else {
             fold();
         }
         c->prof_mark();
-        BfRound rp{};
-        rp.tr = tr; rp.point = point_dev; rp.n_point = n_point; rp.round = round; rp.log_n = log_n;
+        BfRound& rp = rounds.r[round];
         rp.alpha_next = round + 1 < log_n ? alpha + round + 1 : nullptr;
         rp.prev_values = prev_cw; rp.prev_nodes = prev_tree; rp.fold_values = next_cw; rp.fold_nodes = next_tree;
         rp.h_prev = h_prev;
@@ -419,8 +445,11 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
         size_t off = c->rec_alloc(bf_round_words(h_prev));
         rp.rec = c->rec_dev + off;
         pd.round_off.push_back(off);
-        bf_round_kernel<<<1, 256, exclusive_smem(bf_round_kernel, c), c->stream>>>(rp);
-        ZKB_LAUNCHED(c);
+        if (!ahead) {                    // the buffers are used again two rounds later, so the paths are gathered now
+            rounds.first = round; rounds.count = 1;
+            bf_launch_chain(c, rounds);
+            bf_launch_gather(c, rounds);
+        }
         c->prof_mark();
         if (ahead) {
             prev_cw = next_cw; prev_tree = next_tree;
@@ -431,6 +460,15 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
             std::swap(prev_cw, next_cw);
             std::swap(prev_tree, next_tree);
         }
+    }
+    if (ahead) {
+        for (rounds.first = 0; rounds.first < log_n; rounds.first += rounds.count) {
+            rounds.count = bf_chain_rounds(rounds.first, log_n);
+            ZKB_CUDA(cudaStreamWaitEvent(main_stream, c->side_event(rounds.first + rounds.count - 1), 0));
+            bf_launch_chain(c, rounds);
+        }
+        rounds.first = 0; rounds.count = log_n;
+        bf_launch_gather(c, rounds);
     }
     pd.final_off = c->rec_alloc(1);
     ZKB_CUDA(cudaMemcpyAsync(c->rec_dev + pd.final_off, eval, 4, cudaMemcpyDeviceToDevice, c->stream));
