@@ -178,7 +178,9 @@ __device__ __forceinline__ u32 bf_next_alpha(Tr& tr, const u32* point, u32 n_poi
     return tr_squeeze(tr);
 }
 // The transcript's part of some rounds: absorb the folded root, squeeze the query positions, take the next challenge.  This
-// is the opening's critical path, so nothing else is in it: the paths are gathered by bf_gather_kernel, off the chain.
+// is the opening's critical path (26 dependent SHA-256 compressions a round, one thread, about 58 us), so nothing else is in
+// it: the paths are gathered by bf_gather_kernel, off the chain.  Measured on B200 with the gathers inside and a launch per
+// round -> like this: Basefold of 2^24 coefficients 3213 -> 3053 us.
 __global__ void __launch_bounds__(32) bf_chain_kernel(const __grid_constant__ BfRounds a) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     if (threadIdx.x) return;
