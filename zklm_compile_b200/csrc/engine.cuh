@@ -125,11 +125,11 @@ void run_sumcheck(zkb_ctx* c, ScTables tb, u32 num_vars, ScIO io, bool dynamic, 
         pending = true;
         round++;
     }
-    // product sumchecks over EF tables: the tail that overlaps the table work with the hash chain
-    constexpr bool pipe_t = KIND == SC_PRODUCT && std::is_same<ChalT, Fe>::value;
-    const bool pipe = pipe_t && !c->opt_plain_tail && !io.xch && !dynamic && !io.dyn_nv && (!in_src || std::is_same<SrcT, Fe>::value);
+    // product sumchecks whose tables have the challenges' type by now: the tail that overlaps the table work with the hash chain
+    constexpr bool pipe_t = KIND == SC_PRODUCT;
+    const bool pipe = pipe_t && !c->opt_plain_tail && !io.xch && !dynamic && !io.dyn_nv && (!in_src || std::is_same<SrcT, ChalT>::value);
     if (pipe) {
-        if constexpr (pipe_t) sc_tail_product_pipe_kernel<<<1, c->pipe_threads(PIPE_THREADS), 0, c->stream>>>(tb, size, round, num_vars, pending ? 1 : 0, io);
+        if constexpr (pipe_t) sc_tail_product_pipe_kernel<ChalT><<<1, c->pipe_threads(PIPE_THREADS), 0, c->stream>>>(tb, size, round, num_vars, pending ? 1 : 0, io);
     } else if (in_src)
         sc_tail_kernel<KIND, SrcT, ChalT><<<1, c->single_cta_threads(), 0, c->stream>>>(tb, size, round, num_vars, pending ? 1 : 0, io);
     else

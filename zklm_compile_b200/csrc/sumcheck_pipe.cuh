@@ -1,5 +1,6 @@
-// Single-CTA tail of the product sumcheck over EF tables with the table work taken off the
-// critical path (rust/zk_ml_prover/src/proving/sumcheck.rs:1262-1315 computes the same messages).
+// Single-CTA tail of the product sumcheck, over EF tables with EF challenges or over base-field tables with base-field
+// challenges (T = Fe or Fp), with the table work taken off the critical path
+// (rust/zk_ml_prover/src/proving/sumcheck.rs:211-272, 1262-1315 compute the same messages).
 //
 // In the plain tail every round is: pass over the tables (fold with the last challenge, sum the
 // round polynomial), block reduction, then one thread hashes (about five SHA-256 compressions)
@@ -11,6 +12,9 @@
 // evaluates the three quadratics and goes on hashing; the table work overlaps the hash chain
 // instead of alternating with it.  All values are canonical field elements, so the messages are
 // bit-identical to the plain tail's.
+// Base-field rounds hash one compression instead of five, so the table pass and its reduction were most of such a round:
+// measured on B200 with the plain tail -> with this one, a whole op-list proof of the 1024-2048-1024-10 MLP 1676 -> 1579 us,
+// of the 182-op GPT-2 shape 60.6 -> 57.3 ms.
 #pragma once
 #include "sumcheck.cuh"
 
@@ -18,7 +22,7 @@ namespace zkb {
 
 constexpr int PIPE_THREADS = 512;                                 // at most; 128 registers per thread (the worker pass keeps 36 sums)
 constexpr int PIPE_MAX_WORKER_WARPS = PIPE_THREADS / 32 - 1;      // 15
-constexpr int PIPE_NW = 36;                                       // nine EF coefficient sums
+template <class T> constexpr int PIPE_NW = 9 * Width<T>::W;   // nine coefficient sums
 
 // Roles.  Warp 0 hashes.  Warps 4, 8, 12 would share warp 0's scheduler (warp w issues on sub-
 // partition w mod 4), its instruction cache and its issue slots; they only join the CTA barriers,
@@ -31,31 +35,34 @@ __device__ __forceinline__ int pipe_worker_warps() { const int last = (int)(bloc
 __device__ __forceinline__ void pipe_worker_barrier() { asm volatile("bar.sync 1, %0;" ::"r"(pipe_worker_warps() * 32) : "memory"); }
 
 // Coefficient sums of the next round over one pair index: quarters (a, b, c, d) of f and g.
-__device__ __forceinline__ void pipe_accum(Fe* C, Fe fa, Fe fb, Fe fc, Fe fd, Fe ga, Fe gb, Fe gc, Fe gd) {
-    const Fe ef = fb - fa, eg = gb - ga, hf = fd - fc, hg = gd - gc;       // lo = a + r e, hi = c + r h
+template <class T>
+__device__ __forceinline__ void pipe_accum(T* C, T fa, T fb, T fc, T fd, T ga, T gb, T gc, T gd) {
+    const T ef = fb - fa, eg = gb - ga, hf = fd - fc, hg = gd - gc;       // lo = a + r e, hi = c + r h
     C[0] = C[0] + fa * ga;  C[1] = C[1] + fa * eg + ga * ef;  C[2] = C[2] + ef * eg;
     C[3] = C[3] + fc * gc;  C[4] = C[4] + fc * hg + gc * hf;  C[5] = C[5] + hf * hg;
-    const Fe pf = dbl_minus(fc, fa), pg = dbl_minus(gc, ga);               // 2 hi - lo at r = 0
-    const Fe qf = dbl_minus(hf, ef), qg = dbl_minus(hg, eg);               // its slope in r
+    const T pf = dbl_minus(fc, fa), pg = dbl_minus(gc, ga);               // 2 hi - lo at r = 0
+    const T qf = dbl_minus(hf, ef), qg = dbl_minus(hg, eg);               // its slope in r
     C[6] = C[6] + pf * pg;  C[7] = C[7] + pf * qg + pg * qf;  C[8] = C[8] + qf * qg;
 }
 
-// Workers only (see pipe_is_worker; at least two worker warps, so that 36 threads can add the rows).  Tables of size n at (rf, rg); if `fold`, they are first
+// Workers only (see pipe_is_worker; at least two worker warps, so that PIPE_NW threads can add the rows).  Tables of size n at (rf, rg); if `fold`, they are first
 // folded with r into size n / 2 at (wf, wg) (in place allowed) and the sums are taken over the
-// folded tables.  Leaves the 36 summed words in out[] (shared memory) when the result size is >= 4.
-__device__ __forceinline__ void pipe_worker_pass(const Fe* rf, const Fe* rg, Fe* wf, Fe* wg, size_t n, bool fold, Fe r,
-                                                 u32 (*cw)[PIPE_NW], u32* out) {
+// folded tables.  Leaves the PIPE_NW summed words in out[] (shared memory) when the result size is >= 4.
+template <class T>
+__device__ __forceinline__ void pipe_worker_pass(const T* rf, const T* rg, T* wf, T* wg, size_t n, bool fold, T r,
+                                                 u32 (*cw)[PIPE_NW<T>], u32* out) {
+    constexpr int NW = PIPE_NW<T>;
     const int worker_warps = pipe_worker_warps();
     const int wid = pipe_worker_index(threadIdx.x >> 5) * 32 + (threadIdx.x & 31);
     const size_t workers = (size_t)worker_warps * 32;
     const size_t m = fold ? n / 2 : n;              // size of the tables the sums run over
-    Fe C[9];
+    T C[9];
 #pragma unroll
-    for (int i = 0; i < 9; i++) C[i] = fe_zero();
+    for (int i = 0; i < 9; i++) C[i] = zero_of<T>();
     if (m >= 4) {
         const size_t q = m / 4;                     // pair indices of the next round
         for (size_t j = wid; j < q; j += workers) {
-            Fe fa, fb, fc, fd, ga, gb, gc, gd;
+            T fa, fb, fc, fd, ga, gb, gc, gd;
             if (fold) {
                 // folded element x is lerp(T[x], T[x + n/2], r); this thread owns x = j, j+q, j+2q, j+3q
                 const size_t h = n / 2;
@@ -76,27 +83,27 @@ __device__ __forceinline__ void pipe_worker_pass(const Fe* rf, const Fe* rg, Fe*
         if (wid == 0) {
             const size_t h = n / 2;
             for (size_t x = 0; x < h; x++) {
-                Fe a = lerp(ld_fe(rf + x), ld_fe(rf + x + h), r), b = lerp(ld_fe(rg + x), ld_fe(rg + x + h), r);
+                T a = lerp(ld_fe(rf + x), ld_fe(rf + x + h), r), b = lerp(ld_fe(rg + x), ld_fe(rg + x + h), r);
                 st_fe(wf + x, a); st_fe(wg + x, b);
             }
         }
     }
     if (m >= 4) {
-        u32 w[PIPE_NW];
+        u32 w[NW];
 #pragma unroll
-        for (int i = 0; i < 9; i++) to_words(C[i], w + 4 * i);
+        for (int i = 0; i < 9; i++) to_words(C[i], w + Width<T>::W * i);
         const int lane = threadIdx.x & 31, warp = pipe_worker_index(threadIdx.x >> 5);
 #pragma unroll
-        for (int k = 0; k < PIPE_NW; k++) {
+        for (int k = 0; k < NW; k++) {
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) w[k] = add31(w[k], __shfl_down_sync(0xffffffffu, w[k], off));
         }
         if (lane == 0) {
 #pragma unroll
-            for (int k = 0; k < PIPE_NW; k++) cw[warp][k] = w[k];
+            for (int k = 0; k < NW; k++) cw[warp][k] = w[k];
         }
         pipe_worker_barrier();
-        if (wid < PIPE_NW) {
+        if (wid < NW) {
             u32 v = 0;
             for (int rw = 0; rw < worker_warps; rw++) v = add31(v, cw[rw][wid]);
             out[wid] = v;
@@ -104,40 +111,42 @@ __device__ __forceinline__ void pipe_worker_pass(const Fe* rf, const Fe* rg, Fe*
     }
 }
 
+template <class T>
 __global__ void __launch_bounds__(PIPE_THREADS) sc_tail_product_pipe_kernel(ScTables tb, size_t size, u32 round, u32 num_vars,
                                                                                int pending, ScIO io) {
+    constexpr int W = Width<T>::W, NW = PIPE_NW<T>;
     __shared__ u32 red[32 * 16];
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
-    __shared__ u32 r_sh[2][4];                       // indexed by round parity: round k+1's challenge never overwrites r_k while a slow warp still reads it
-    __shared__ u32 cw[PIPE_MAX_WORKER_WARPS][PIPE_NW];
-    __shared__ u32 csum[2][PIPE_NW];
-    __shared__ u32 w_sh[12];
+    __shared__ u32 r_sh[2][W];                       // indexed by round parity: round k+1's challenge never overwrites r_k while a slow warp still reads it
+    __shared__ u32 cw[PIPE_MAX_WORKER_WARPS][NW];
+    __shared__ u32 csum[2][NW];
+    __shared__ u32 w_sh[3 * W];
 
     ZKB_STAMP_BEGIN
     Tr tr;
     if (threadIdx.x == 0) tr_load(tr, io.tr, trbuf);
-    Fe r = fe_zero();
-    if (pending) from_words(r, io.chal + (size_t)(round - 1) * 4);
+    T r = zero_of<T>();
+    if (pending) from_words(r, io.chal + (size_t)(round - 1) * W);
 
     // ---- prologue: the message of `round`, computed directly by the whole CTA
-    const Fe* rf = reinterpret_cast<const Fe*>(tb.src[0]);
-    const Fe* rg = reinterpret_cast<const Fe*>(tb.src[1]);
-    Fe* wf = reinterpret_cast<Fe*>(tb.dst[0]);
-    Fe* wg = reinterpret_cast<Fe*>(tb.dst[1]);
+    const T* rf = reinterpret_cast<const T*>(tb.src[0]);
+    const T* rg = reinterpret_cast<const T*>(tb.src[1]);
+    T* wf = reinterpret_cast<T*>(tb.dst[0]);
+    T* wg = reinterpret_cast<T*>(tb.dst[1]);
     size_t n = size;                                 // size of the tables the current round sums over
     u32 w[16];
     {
-        Fe acc[3] = {fe_zero(), fe_zero(), fe_zero()};
+        T acc[3] = {zero_of<T>(), zero_of<T>(), zero_of<T>()};
         if (pending) {
-            sc_pass<SC_PRODUCT, Fe, Fe, true>(tb, n / 4, r, threadIdx.x, blockDim.x, acc);
+            sc_pass<SC_PRODUCT, T, T, true>(tb, n / 4, r, threadIdx.x, blockDim.x, acc);
             n /= 2;
             rf = wf; rg = wg;                        // folded tables live in dst from now on
         } else {
-            sc_pass<SC_PRODUCT, Fe, Fe, false>(tb, n / 2, r, threadIdx.x, blockDim.x, acc);
+            sc_pass<SC_PRODUCT, T, T, false>(tb, n / 2, r, threadIdx.x, blockDim.x, acc);
         }
 #pragma unroll
-        for (int k = 0; k < 3; k++) to_words(acc[k], w + 4 * k);
-        block_sum_words<12>(w, red);                 // ends with a CTA barrier: folded tables visible
+        for (int k = 0; k < 3; k++) to_words(acc[k], w + W * k);
+        block_sum_words<3 * W>(w, red);                 // ends with a CTA barrier: folded tables visible
     }
 
     bool first = true;
@@ -145,7 +154,7 @@ __global__ void __launch_bounds__(PIPE_THREADS) sc_tail_product_pipe_kernel(ScTa
     for (;;) {
         // thread 0 hashes round k; the workers prepare round k + 1 as polynomials in r_k
         if (threadIdx.x == 0) {
-            Fe rn = sc_finish_round<SC_PRODUCT, Fe, Fe>(w, io, k, tr);
+            T rn = sc_finish_round<SC_PRODUCT, T, T>(w, io, k, tr);
             to_words(rn, r_sh[k & 1]);
         } else if (pipe_is_worker(threadIdx.x >> 5)) {
             if (first) pipe_worker_pass(rf, rg, wf, wg, n, false, r, cw, csum[k & 1]);
@@ -158,15 +167,15 @@ __global__ void __launch_bounds__(PIPE_THREADS) sc_tail_product_pipe_kernel(ScTa
         if (n == 2) break;                           // round k was the last one
         if (threadIdx.x < 32) {                      // three lanes evaluate the three quadratics, lane 0 collects
             if (threadIdx.x < 3) {
-                const u32* c = csum[k & 1] + 12 * threadIdx.x;
-                Fe c0, c1, c2;
-                from_words(c0, c); from_words(c1, c + 4); from_words(c2, c + 8);
-                to_words(c0 + r * (c1 + r * c2), w_sh + 4 * threadIdx.x);
+                const u32* c = csum[k & 1] + 3 * W * threadIdx.x;
+                T c0, c1, c2;
+                from_words(c0, c); from_words(c1, c + W); from_words(c2, c + 2 * W);
+                to_words(c0 + r * (c1 + r * c2), w_sh + W * threadIdx.x);
             }
             __syncwarp();
             if (threadIdx.x == 0) {
 #pragma unroll
-                for (int i = 0; i < 12; i++) w[i] = w_sh[i];
+                for (int i = 0; i < 3 * W; i++) w[i] = w_sh[i];
             }
         }
         k++;
@@ -181,9 +190,9 @@ __global__ void __launch_bounds__(PIPE_THREADS) sc_tail_product_pipe_kernel(ScTa
         }
         tr_store(tr, io.tr);
         // two elements per table remain (folded through r_(k-1)): fold the last challenge in
-        Fe fv = lerp(ld_fe(rf), ld_fe(rf + 1), r), gv = lerp(ld_fe(rg), ld_fe(rg + 1), r);
+        T fv = lerp(ld_fe(rf), ld_fe(rf + 1), r), gv = lerp(ld_fe(rg), ld_fe(rg + 1), r);
         to_words(fv, io.fin);
-        to_words(gv, io.fin + 4);
+        to_words(gv, io.fin + W);
     }
     ZKB_STAMP_END(io.tr, 1);
 }
