@@ -82,6 +82,24 @@ def test_sumcheck_matches_oracle(ctx, kind, nv):
     assert tr.squeeze() == otr.squeeze()
 
 
+@pytest.mark.parametrize("kind", [zk.SC_PRODUCT_EF, zk.SC_PRODUCT_EF_FULL, zk.SC_PRODUCT_EF_MIXED])
+@pytest.mark.parametrize("nv", [14, 16, 17, 19])
+def test_launches_of_two_rounds_match_oracle(ctx, kind, nv):
+    """Around the size at which rounds 0 and 1 of base tables begin to share a launch (2^15), with and without rounds between
+    the two-challenge fold and the tail; the extension-field kinds keep a launch per round."""
+    tables = rand_tables(kind, nv, 5000 * kind + nv)
+    dev = [ctx.upload(t) for t in tables]
+    tr, otr = zk.Transcript(ctx, b"two"), O.Transcript(b"two")
+    proof, *fin = zk.sumcheck_prove(kind, dev, nv, tr)
+    polys, chal, ofin = O.prove(KIND_NAMES[kind], otr, tables, nv)
+    assert proof.round_polys.reshape(nv, -1).tolist() == polys.tolist()
+    assert proof.challenges.reshape(nv, -1).tolist() == chal.tolist()
+    assert np.array([np.asarray(f, dtype=np.uint32).reshape(-1) for f in fin]).tolist() == ofin.tolist()
+    assert tr.squeeze() == otr.squeeze()
+    for d, t in zip(dev, tables):
+        assert np.array_equal(d.download().reshape(t.shape), t)
+
+
 @pytest.mark.parametrize("kind", [zk.SC_PRODUCT_EF, zk.SC_PRODUCT, zk.SC_TRIPLE_EF_FULL])
 def test_sumcheck_device_tables_untouched_and_verifies(ctx, kind):
     nv = 14

@@ -76,6 +76,33 @@ void run_sumcheck(zkb_ctx* c, ScTables tb, u32 num_vars, ScIO io, bool dynamic, 
     const int max_grid = c->sm_count * per_sm < SC_MAX_GRID ? c->sm_count * per_sm : SC_MAX_GRID;
     c->prof_used = 0;
     c->prof_mark();
+    auto launch_fold2 = [&] {                    // both pending challenges folded in, tables shrink to a quarter
+        const size_t E = size / 8;
+        const int vec = c->opt_fold2_vec ? c->opt_fold2_vec : 2;
+        const size_t want2 = (E / vec + 255) / 256;
+        const int g2 = (int)(want2 < (size_t)max_grid ? want2 : (size_t)max_grid);
+        if (vec == 1) sc_product_base_fold2_kernel<1><<<g2, 256, 0, c->stream>>>(tb, E, round, io);
+        else if (vec == 4) sc_product_base_fold2_kernel<4><<<g2, 256, 0, c->stream>>>(tb, E, round, io);
+        else sc_product_base_fold2_kernel<2><<<g2, 256, 0, c->stream>>>(tb, E, round, io);
+    };
+    if constexpr (KIND == SC_PRODUCT && std::is_same<SrcT, Fp>::value && std::is_same<ChalT, Fe>::value) {
+        // Every round on this GPU: rounds 0 and 1 share a launch.  (Split over several GPUs, each round's sums are exchanged.)
+        if (fused2 && !dynamic && !io.xch) {
+            const size_t vcap = c->polite ? (size_t)c->sm_count : (size_t)max_grid, want = (size / 16 + 255) / 256;
+            sc_product_base_two_kernel<<<(int)(want < vcap ? want : vcap), 256, 0, c->stream>>>(tb, size / 4, round, io);
+            ZKB_LAUNCHED(c);
+            c->prof_mark();
+            round += 2;
+            launch_fold2();
+            ZKB_LAUNCHED(c);
+            c->prof_mark();
+            for (int t = 0; t < 3; t++) tb.src[t] = tb.dst[t];
+            in_src = false;
+            pending = true;
+            size /= 4;
+            round++;
+        }
+    }
     while (!dynamic && round < local_vars) {
         size_t half = pending ? size / 4 : size / 2;
         if (half < MULTI_MIN_HALF) break;
@@ -101,13 +128,7 @@ void run_sumcheck(zkb_ctx* c, ScTables tb, u32 num_vars, ScIO io, bool dynamic, 
                     ZKB_LAUNCHED(c);
                     c->prof_mark();
                     round++;
-                    const size_t E = size / 8;
-                    const int vec = c->opt_fold2_vec ? c->opt_fold2_vec : 2;
-                    const size_t want2 = (E / vec + 255) / 256;
-                    const int g2 = (int)(want2 < (size_t)max_grid ? want2 : (size_t)max_grid);
-                    if (vec == 1) sc_product_base_fold2_kernel<1><<<g2, 256, 0, c->stream>>>(tb, E, round, io);
-                    else if (vec == 4) sc_product_base_fold2_kernel<4><<<g2, 256, 0, c->stream>>>(tb, E, round, io);
-                    else sc_product_base_fold2_kernel<2><<<g2, 256, 0, c->stream>>>(tb, E, round, io);
+                    launch_fold2();
                     size /= 2;                          // two folds in all: one here, one below
                     done = true;
                 } else if (base_product) { sc_product_base_kernel<Fe, true><<<vgrid, 256, 0, c->stream>>>(tb, half, round, io); done = true; }

@@ -257,6 +257,21 @@ __device__ __forceinline__ void ld4(const void* base, size_t j, u32* o) {
 
 // WRITE = false (with FOLD): the folded tables are not materialised - the launch only produces
 // the round message (the fused launch below folds two challenges at once from the base tables).
+__device__ __forceinline__ void sc_base_coef_accum(u64* acc, u32 fa, u32 fb, u32 fc, u32 fd, u32 ga, u32 gb, u32 gc, u32 gd) {
+    const u32 ef = sub31(fb, fa), eg = sub31(gb, ga);       // lo = a + r e
+    const u32 hf = sub31(fd, fc), hg = sub31(gd, gc);       // hi = c + r h
+    acc[0] += fold62((u64)fa * ga);
+    acc[1] += fold62((u64)fa * eg + (u64)ga * ef);
+    acc[2] += fold62((u64)ef * eg);
+    acc[3] += fold62((u64)fc * gc);
+    acc[4] += fold62((u64)fc * hg + (u64)gc * hf);
+    acc[5] += fold62((u64)hf * hg);
+    const u32 pf = sub31(add31(fc, fc), fa), pg = sub31(add31(gc, gc), ga);   // 2 hi - lo at r = 0
+    const u32 qf = sub31(add31(hf, hf), ef), qg = sub31(add31(hg, hg), eg);   // its slope in r
+    acc[6] += fold62((u64)pf * pg);
+    acc[7] += fold62((u64)pf * qg + (u64)pg * qf);
+    acc[8] += fold62((u64)qf * qg);
+}
 template <class ChalT, bool FOLD, bool WRITE = true>
 __global__ void __launch_bounds__(256) sc_product_base_kernel(ScTables tb, size_t half, u32 round, ScIO io) {
     constexpr int NACC = FOLD ? 9 : 3;
@@ -288,9 +303,9 @@ __global__ void __launch_bounds__(256) sc_product_base_kernel(ScTables tb, size_
             ld4(tb.src[1], j, ga); ld4(tb.src[1], j + 2 * half, gb); ld4(tb.src[1], j + half, gc); ld4(tb.src[1], j + 3 * half, gd);
 #pragma unroll
             for (int v = 0; v < 4; v++) {
-                const u32 ef = sub31(fb[v], fa[v]), eg = sub31(gb[v], ga[v]);       // lo = a + r e
-                const u32 hf = sub31(fd[v], fc[v]), hg = sub31(gd[v], gc[v]);       // hi = c + r h
                 if constexpr (WRITE) {      // folded tables (EF = base + r * base)
+                    const u32 ef = sub31(fb[v], fa[v]), eg = sub31(gb[v], ga[v]);       // lo = a + r e
+                    const u32 hf = sub31(fd[v], fc[v]), hg = sub31(gd[v], gc[v]);       // hi = c + r h
                     Fe lf = r * Fp{ef}; lf.x = add31(lf.x, fa[v]);
                     Fe lg = r * Fp{eg}; lg.x = add31(lg.x, ga[v]);
                     Fe uf = r * Fp{hf}; uf.x = add31(uf.x, fc[v]);
@@ -298,18 +313,7 @@ __global__ void __launch_bounds__(256) sc_product_base_kernel(ScTables tb, size_
                     st_el<Fe>(tb.dst[0], j + v, lf); st_el<Fe>(tb.dst[0], j + half + v, uf);
                     st_el<Fe>(tb.dst[1], j + v, lg); st_el<Fe>(tb.dst[1], j + half + v, ug);
                 }
-                // coefficient sums
-                acc[0] += fold62((u64)fa[v] * ga[v]);
-                acc[1] += fold62((u64)fa[v] * eg + (u64)ga[v] * ef);
-                acc[2] += fold62((u64)ef * eg);
-                acc[3] += fold62((u64)fc[v] * gc[v]);
-                acc[4] += fold62((u64)fc[v] * hg + (u64)gc[v] * hf);
-                acc[5] += fold62((u64)hf * hg);
-                const u32 pf = sub31(add31(fc[v], fc[v]), fa[v]), pg = sub31(add31(gc[v], gc[v]), ga[v]);   // 2 hi - lo at r = 0
-                const u32 qf = sub31(add31(hf, hf), ef), qg = sub31(add31(hg, hg), eg);                     // its slope in r
-                acc[6] += fold62((u64)pf * pg);
-                acc[7] += fold62((u64)pf * qg + (u64)pg * qf);
-                acc[8] += fold62((u64)qf * qg);
+                sc_base_coef_accum(acc, fa[v], fb[v], fc[v], fd[v], ga[v], gb[v], gc[v], gd[v]);
             }
         }
     }
@@ -444,6 +448,70 @@ __global__ void __launch_bounds__(256) sc_product_base_fold2_kernel(ScTables tb,
         Tr tr;
         tr_load(tr, io.tr, trbuf);
         sc_finish_round<SC_PRODUCT, Fe, Fe>(t, io, round, tr);
+        tr_store(tr, io.tr);
+        *io.counter = 0;
+    }
+}
+
+// ---- product sumcheck over base-field tables: rounds 0 and 1 in one launch -------------------------------
+// The nine coefficient sums of round 1 determine round 0 as well: with quarters (a, b, c, d) of the tables, s(0) = sum (a a +
+// c c) = A0 + C0, s(1) is both quadratics at r = 1 and s(2) both at r = 2.  So one pass over the tables serves both
+// rounds: the finishing CTA hashes the first message, evaluates the quadratics at the challenge and hashes the second.  The
+// launch is bound by HBM (it reads 8 N bytes, N elements to a table); a launch for each round read them twice.
+// (Two rounds per launch on the extension-field tables behind it move 37 N bytes in all instead of 48 N, but there
+// a pair costs nine EF products, about 2600 issue slots of field reductions with the folds: bound by those, not kept.)
+// `q` = a quarter of the tables' length, a multiple of four.
+__global__ void __launch_bounds__(256) sc_product_base_two_kernel(ScTables tb, size_t q, u32 round, ScIO io) {
+    __shared__ u32 red[32 * 16];
+    __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
+    __shared__ bool is_last;
+    u64 acc[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) acc[k] = 0;
+    const size_t stride = (size_t)gridDim.x * blockDim.x * 4;
+    for (size_t j = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; j < q; j += stride) {
+        u32 fa[4], fb[4], fc[4], fd[4], ga[4], gb[4], gc[4], gd[4];
+        ld4(tb.src[0], j, fa); ld4(tb.src[0], j + 2 * q, fb); ld4(tb.src[0], j + q, fc); ld4(tb.src[0], j + 3 * q, fd);
+        ld4(tb.src[1], j, ga); ld4(tb.src[1], j + 2 * q, gb); ld4(tb.src[1], j + q, gc); ld4(tb.src[1], j + 3 * q, gd);
+#pragma unroll
+        for (int v = 0; v < 4; v++) sc_base_coef_accum(acc, fa[v], fb[v], fc[v], fd[v], ga[v], gb[v], gc[v], gd[v]);
+    }
+    u32 w[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) w[k] = red64(acc[k]);
+    block_sum_words<9>(w, red);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < 9; k++) io.partials[(size_t)blockIdx.x * 16 + k] = w[k];
+        __threadfence();
+        unsigned int ticket = atomicAdd(io.counter, 1u);
+        is_last = (ticket == gridDim.x - 1);
+    }
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    u32 t[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) t[k] = 0;
+    for (u32 b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
+#pragma unroll
+        for (int k = 0; k < 9; k++) t[k] = add31(t[k], __ldcg(io.partials + (size_t)b * 16 + k));
+    }
+    block_sum_words<9>(t, red);
+    if (threadIdx.x == 0) {
+        Tr tr;
+        tr_load(tr, io.tr, trbuf);
+        const u32 l0 = add31(t[0], t[3]), l1 = add31(t[1], t[4]), l2 = add31(t[2], t[5]);
+        const u32 m0[3] = {l0, add31(l0, add31(l1, l2)), add31(l0, add31(add31(l1, l1), mul31(4u, l2)))};
+        const Fe r = sc_finish_round<SC_PRODUCT, Fp, Fe>(m0, io, round, tr), r2 = r * r;
+        u32 m1[12];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            Fe s = r * Fp{t[3 * k + 1]} + r2 * Fp{t[3 * k + 2]};
+            s.x = add31(s.x, t[3 * k]);
+            to_words(s, m1 + 4 * k);
+        }
+        sc_finish_round<SC_PRODUCT, Fe, Fe>(m1, io, round + 1, tr);
         tr_store(tr, io.tr);
         *io.counter = 0;
     }
