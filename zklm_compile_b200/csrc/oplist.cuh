@@ -138,7 +138,7 @@ __global__ void layernorm_prep_kernel(const u32* __restrict__ xc, const u32* __r
 __global__ void __launch_bounds__(TRSCRIPT_THREADS) hash_values_kernel(const u32* __restrict__ v, u32 n, u32* digest_out) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     __shared__ u32 tile[2 * 512];
-    __shared__ u32 kw[2 * 32 * SHA_KW_STRIDE];
+    __shared__ __align__(16) u32 kw[2 * 32 * SHA_KW_STRIDE];
     __shared__ u32 bc[1];
     Tr tr;
     tr.buf = trbuf; tr.buflen = 0; tr.total = 0;
@@ -158,7 +158,7 @@ struct HashJob { const u32* v; u32 n; u32 _pad; };
 __global__ void __launch_bounds__(TRSCRIPT_THREADS) hash_values_multi_kernel(const HashJob* __restrict__ jobs, u32* digests_out) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     __shared__ u32 tile[2 * 512];
-    __shared__ u32 kw[2 * 32 * SHA_KW_STRIDE];
+    __shared__ __align__(16) u32 kw[2 * 32 * SHA_KW_STRIDE];
     __shared__ u32 bc[1];
     const u32* v = jobs[blockIdx.x].v;
     const u32 n = jobs[blockIdx.x].n;

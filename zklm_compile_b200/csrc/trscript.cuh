@@ -29,7 +29,7 @@ __global__ void tr_absorb_bytes_kernel(TrState* st, ByteChunk c, u32 n) {
 __global__ void __launch_bounds__(32) tr_absorb_words_kernel(TrState* st, const u32* __restrict__ v, size_t n) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     __shared__ u32 tile[512];
-    __shared__ u32 kw[32 * SHA_KW_STRIDE];
+    __shared__ __align__(16) u32 kw[32 * SHA_KW_STRIDE];
     Tr tr;
     tr.buf = trbuf; tr.buflen = 0; tr.total = 0;
     if (threadIdx.x == 0) tr_load(tr, st, trbuf);
@@ -75,7 +75,7 @@ constexpr int TRSCRIPT_THREADS = 64;      // warp 0 advances the transcript, war
 __global__ void __launch_bounds__(TRSCRIPT_THREADS) tr_script_kernel(TrState* st, TrScript sc) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     __shared__ u32 tile[2 * 512];
-    __shared__ u32 kw[2 * 32 * SHA_KW_STRIDE];
+    __shared__ __align__(16) u32 kw[2 * 32 * SHA_KW_STRIDE];
     __shared__ u32 bc[1];
     ZKB_STAMP_BEGIN
     Tr tr;
