@@ -80,6 +80,27 @@ def test_device_resident_polynomials_and_in_order_schedule(ctx):
     b.close()
 
 
+def test_calls_behind_a_batch_that_exhausts_the_record_buffer(ctx):
+    """1100 joining polynomials have more opened paths than the record buffer holds: the call returns a status while folds and trees
+    of the large polynomial are still running on the second stream, and what comes next on the context must not meet them."""
+    rng = np.random.default_rng(31)
+    big, small, n = rng.integers(0, P, 1 << 21).astype(np.uint32), rng.integers(0, P, 1 << 10).astype(np.uint32), (1 << 17) - 3
+    coeffs, point = rng.integers(0, P, n).astype(np.uint32), rng.integers(0, P, 17).astype(np.uint32)
+    b = pcs.BasefoldBatch(ctx, [big] + [small] * 1100, [21] + [10] * 1100)
+    ok = pcs.BasefoldBatch(ctx, [coeffs, small], [17, 10])
+    exp = [O.basefold_commit_and_prove(O.Transcript(b"behind"), coeffs, point, 0), O.basefold_batch_prove(O.Transcript(b"behind"), [coeffs, small], [17, 10])]
+    trs = [zk.Transcript(ctx, b"behind") for _ in range(4)]
+    for t in (0, 2):
+        with pytest.raises(zk.ZkbError, match="record buffer exhausted") as e:
+            b.prove(trs[t])
+        assert e.value.code == 7
+        got = [pcs.basefold_commit_and_prove(ctx, trs[t + 1], coeffs, point), None]
+        got[1] = ok.prove(zk.Transcript(ctx, b"behind"))
+        assert got == exp
+    b.close()
+    ok.close()
+
+
 def test_argument_errors(ctx):
     p = np.arange(10, dtype=np.uint32)
     with pytest.raises(zk.ZkbError):

@@ -139,12 +139,7 @@ BfbPending bfb_enqueue(zkb_bf_batch* B, TrState* tr, bool individual) {
     ZKB_LAUNCHED(c);
 
     const bool in_order = c->opt_bf_in_order || c->capturing;
-    cudaStream_t main_stream = c->stream, work = in_order ? main_stream : c->side_stream();
-    if (!in_order) {
-        cudaEvent_t fork = c->side_event(log_n);
-        ZKB_CUDA(cudaEventRecord(fork, main_stream));
-        ZKB_CUDA(cudaStreamWaitEvent(work, fork, 0));
-    }
+    SideFork fork(c, !in_order, log_n);
     // final value: sum_i rho^i MLE_i(fold_point[..log_n_i]) (:1357-1362).  It needs only the fold point, so it goes in front of the rounds on
     // the main stream, where it runs while the second stream folds and hashes the first (largest) rounds.
     u32* evals = (u32*)c->scratch((size_t)k * 4 + 16);
@@ -172,47 +167,46 @@ BfbPending bfb_enqueue(zkb_bf_batch* B, TrState* tr, bool individual) {
         f.w_len = size_t(1) << fold_level;
         f.prev_partner = round == 0 ? 0 : half;
         f.alpha = fold_point + round;
-        c->stream = work;
-        try {
-            // codewords that reach their own length at this round join the chain (:1304-1314); a codeword of 2 * 2^target values
-            // is exactly as long as the folded one, and its two halves are the same
-            u32 first = 0, count = 0;
-            while (next_group < groups.size() && groups[next_group].log_n == target) {
-                if (!count) first = groups[next_group].s;
-                count += groups[next_group].e - groups[next_group].s;
-                next_group++;
-            }
-            if (count) {
-                u32* add = (u32*)c->scratch(half / 2 * 4 + 16);
-                const size_t len = bfb_vec_len(half / 2);
-                bfb_lincomb_kernel<<<grid_for(c, len / 4), 256, 0, c->stream>>>(B->cw_ptrs_dev, coef, first, count, len, add);
-                ZKB_LAUNCHED(c);
-                f.add = add;
-                f.add_mask = half / 2 - 1;
-            }
-            if (!reuse) mk_build(c, kind, MK_FOLD, nullptr, half, h_prev - 1, next_tree, f);
-            c->stream = main_stream;
-            if (!in_order) ZKB_CUDA(cudaEventRecord(c->side_event(round), work));
-            BfRound& rp = rounds.r[round];
-            rp.alpha_next = round + 1 < log_n ? fold_point + log_n : nullptr;    // the value is already in fold_point; the slot behind it takes the copy
-            rp.prev_values = prev_cw; rp.prev_nodes = prev_tree; rp.fold_values = next_cw; rp.fold_nodes = next_tree;
-            rp.h_prev = h_prev;
-            rp.prev_doubled = round == 0;
-            const size_t off = c->rec_alloc(bf_round_words(h_prev));
-            rp.rec = c->rec_dev + off;
-            pd.round_off.push_back(off);
-            // the joined polynomials' own trees are opened at this round's positions (:1330-1345)
-            for (u32 i = first; i < first + count; i++)
-                pd.add_opens.push_back(BfbPending::Open{round, i, c->rec_alloc(2 * (size_t)BF_QUERIES * (2 + 4 * (size_t)B->e[i].log_n))});
-        } catch (...) { c->stream = main_stream; throw; }
+        // codewords that reach their own length at this round join the chain (:1304-1314); a codeword of 2 * 2^target values
+        // is exactly as long as the folded one, and its two halves are the same
+        c->stream = fork.side;
+        u32 first = 0, count = 0;
+        while (next_group < groups.size() && groups[next_group].log_n == target) {
+            if (!count) first = groups[next_group].s;
+            count += groups[next_group].e - groups[next_group].s;
+            next_group++;
+        }
+        if (count) {
+            u32* add = (u32*)c->scratch(half / 2 * 4 + 16);
+            const size_t len = bfb_vec_len(half / 2);
+            bfb_lincomb_kernel<<<grid_for(c, len / 4), 256, 0, c->stream>>>(B->cw_ptrs_dev, coef, first, count, len, add);
+            ZKB_LAUNCHED(c);
+            f.add = add;
+            f.add_mask = half / 2 - 1;
+        }
+        if (!reuse) mk_build(c, kind, MK_FOLD, nullptr, half, h_prev - 1, next_tree, f);
+        c->stream = fork.main;
+        if (!in_order) ZKB_CUDA(cudaEventRecord(c->side_event(round), fork.side));
+        BfRound& rp = rounds.r[round];
+        rp.alpha_next = round + 1 < log_n ? fold_point + log_n : nullptr;    // the value is already in fold_point; the slot behind it takes the copy
+        rp.prev_values = prev_cw; rp.prev_nodes = prev_tree; rp.fold_values = next_cw; rp.fold_nodes = next_tree;
+        rp.h_prev = h_prev;
+        rp.prev_doubled = round == 0;
+        const size_t off = c->rec_alloc(bf_round_words(h_prev));
+        rp.rec = c->rec_dev + off;
+        pd.round_off.push_back(off);
+        // the joined polynomials' own trees are opened at this round's positions (:1330-1345)
+        for (u32 i = first; i < first + count; i++)
+            pd.add_opens.push_back(BfbPending::Open{round, i, c->rec_alloc(2 * (size_t)BF_QUERIES * (2 + 4 * (size_t)B->e[i].log_n))});
         prev_cw = next_cw; prev_tree = next_tree;
     }
     // every round has buffers of its own, so the chain runs through and the paths of all rounds are gathered behind it
     for (rounds.first = 0; rounds.first < log_n; rounds.first += rounds.count) {
         rounds.count = in_order ? log_n : bf_chain_rounds(rounds.first, log_n);
-        if (!in_order) ZKB_CUDA(cudaStreamWaitEvent(main_stream, c->side_event(rounds.first + rounds.count - 1), 0));
+        if (!in_order) ZKB_CUDA(cudaStreamWaitEvent(fork.main, c->side_event(rounds.first + rounds.count - 1), 0));
         bf_launch_chain(c, rounds);
     }
+    fork.joined();
     rounds.first = 0; rounds.count = log_n;
     bf_launch_gather(c, rounds);
     for (const BfbPending::Open& o : pd.add_opens) {

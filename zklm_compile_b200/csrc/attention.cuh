@@ -479,15 +479,10 @@ inline AttRun attention_prove_enqueue(zkb_ctx* c, TrState* tr, const u32* q, con
     AttArgs F{q, k, v, table_out, n_table, attn_out, R.bind, nullptr, c->status, 0, hpg, gqa};
     att_launch(c, c->stream, F, R.L, R.rows);
     ZKB_CUDA(cudaMemcpyAsync(host_bind, R.bind, (size_t)R.rows * (S + D) * 4, cudaMemcpyDeviceToHost, c->stream));
-    cudaStream_t rows_stream = in_order ? c->stream : c->side_stream();
-    if (!in_order) {
-        ZKB_CUDA(cudaEventRecord(c->side_event(0), c->stream));
-        ZKB_CUDA(cudaStreamWaitEvent(rows_stream, c->side_event(0), 0));
-    }
+    SideFork fork(c, !in_order, 0);
     AttArgs A{q, k, v, table_out, n_table, nullptr, nullptr, R.rec, c->status, 1, hpg, gqa};
-    att_launch(c, rows_stream, A, R.L, R.rows);
-    ZKB_CUDA(cudaMemcpyAsync(host_rec, R.rec, (size_t)R.rows * R.L.words * 4, cudaMemcpyDeviceToHost, rows_stream));
-    if (!in_order) ZKB_CUDA(cudaEventRecord(c->side_event(1), rows_stream));
+    att_launch(c, fork.side, A, R.L, R.rows);
+    ZKB_CUDA(cudaMemcpyAsync(host_rec, R.rec, (size_t)R.rows * R.L.words * 4, cudaMemcpyDeviceToHost, fork.side));
     {   // the dimensions, then every row's scores and outputs (attention.rs:140-143, 254-265)
         ScriptBuilder sb;
         sb.word(num_heads);
@@ -496,7 +491,7 @@ inline AttRun attention_prove_enqueue(zkb_ctx* c, TrState* tr, const u32* q, con
         sb.words_dev(R.bind, (u32)((size_t)R.rows * (S + D)));
         sb.run(c, tr);
     }
-    if (!in_order) ZKB_CUDA(cudaStreamWaitEvent(c->stream, c->side_event(1), 0));
+    fork.join();
     return R;
 }
 

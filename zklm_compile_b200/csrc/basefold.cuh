@@ -462,13 +462,7 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
     none.doubled = 1;
     mk_build(c, kind, MK_VALUES, cwA, n_pad, log_n, treeA, none);
     c->prof_mark();
-    cudaStream_t main_stream = c->stream, side = nullptr;
-    if (ahead) {
-        side = c->side_stream();
-        cudaEvent_t fork = c->side_event(log_n);
-        ZKB_CUDA(cudaEventRecord(fork, main_stream));
-        ZKB_CUDA(cudaStreamWaitEvent(side, fork, 0));
-    }
+    SideFork fork(c, ahead, log_n);
     pd.root_off = c->rec_alloc(4);
     bf_begin_kernel<<<1, 1, 0, c->stream>>>(tr, treeA + mk_node_count(log_n), point_dev, n_point, alpha, c->rec_dev + pd.root_off);
     ZKB_LAUNCHED(c);
@@ -494,14 +488,10 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
                 ZKB_LAUNCHED(c);
             } else mk_build(c, kind, MK_FOLD, nullptr, half, h_prev - 1, next_tree, f);
         };
-        if (ahead) {
-            c->stream = side;
-            try { fold(); } catch (...) { c->stream = main_stream; throw; }
-            c->stream = main_stream;
-            ZKB_CUDA(cudaEventRecord(c->side_event(round), side));
-        } else {
-            fold();
-        }
+        c->stream = fork.side;
+        fold();
+        c->stream = fork.main;
+        if (ahead) ZKB_CUDA(cudaEventRecord(c->side_event(round), fork.side));
         c->prof_mark();
         BfRound& rp = rounds.r[round];
         rp.alpha_next = round + 1 < log_n ? alpha + round + 1 : nullptr;
@@ -530,9 +520,10 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
     if (ahead) {
         for (rounds.first = 0; rounds.first < log_n; rounds.first += rounds.count) {
             rounds.count = bf_chain_rounds(rounds.first, log_n);
-            ZKB_CUDA(cudaStreamWaitEvent(main_stream, c->side_event(rounds.first + rounds.count - 1), 0));
+            ZKB_CUDA(cudaStreamWaitEvent(fork.main, c->side_event(rounds.first + rounds.count - 1), 0));
             bf_launch_chain(c, rounds);
         }
+        fork.joined();
         rounds.first = 0; rounds.count = log_n;
         bf_launch_gather(c, rounds);
     }

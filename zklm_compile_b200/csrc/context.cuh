@@ -250,3 +250,42 @@ struct zkb_transcript {
     zkb_ctx* ctx;
     zkb::TrState* dev;
 };
+
+namespace zkb {
+
+// A stretch of a call that uses the context's second stream beside `stream`: the second one starts behind what `stream` holds,
+// and `stream` waits for it at the end.  Leaving the stretch by an exception joins as well and gives the context its stream
+// back: a call that returns a status must leave nothing running that the next one, which may hand out the same arena memory, is
+// not ordered behind.  Without a fork (`forked` false) `side` is the context's stream and nothing is recorded.
+struct SideFork {
+    zkb_ctx* const c;
+    const cudaStream_t main;
+    cudaStream_t side;
+    SideFork(zkb_ctx* ctx, bool forked, size_t event_index) : c(ctx), main(ctx->stream), side(ctx->stream) {
+        if (!forked) return;
+        side = c->side_stream();
+        ev = c->side_event(event_index);
+        ZKB_CUDA(cudaEventRecord(ev, main));
+        ZKB_CUDA(cudaStreamWaitEvent(side, ev, 0));
+        open = true;
+    }
+    SideFork(const SideFork&) = delete;
+    SideFork& operator=(const SideFork&) = delete;
+    void join() {
+        if (!open) return;
+        ZKB_CUDA(cudaEventRecord(ev, side));
+        ZKB_CUDA(cudaStreamWaitEvent(main, ev, 0));
+        open = false;
+    }
+    void joined() { open = false; }      // the caller's own events have made `main` wait for all of it
+    ~SideFork() {
+        c->stream = main;
+        if (open && (cudaEventRecord(ev, side) != cudaSuccess || cudaStreamWaitEvent(main, ev, 0) != cudaSuccess)) cudaStreamSynchronize(side);
+    }
+
+private:
+    cudaEvent_t ev = nullptr;
+    bool open = false;
+};
+
+}  // namespace zkb

@@ -265,25 +265,16 @@ inline BvRun basefold_verify_enqueue(zkb_ctx* c, TrState* tr, const BvParsed& pr
     ZKB_CUDA(cudaMemcpyAsync(trees, pr.trees.data(), pr.trees.size() * sizeof(BvTree), cudaMemcpyHostToDevice, c->stream));
     ZKB_CUDA(cudaMemsetAsync(run.result_dev, 0, (size_t)run.n_results * 4, c->stream));
     // the Merkle checks need only the proof: second stream, joined before the results are read
-    cudaStream_t main_stream = c->stream, side = c->capturing ? main_stream : c->side_stream();
-    if (side != main_stream) {
-        cudaEvent_t fork = c->side_event(0);
-        ZKB_CUDA(cudaEventRecord(fork, main_stream));
-        ZKB_CUDA(cudaStreamWaitEvent(side, fork, 0));
-    }
-    if (kind == NODE_AES_MMO) bf_verify_batch_kernel<NODE_AES_MMO><<<n_trees, 128, 0, side>>>(words, trees, run.result_dev);
-    else bf_verify_batch_kernel<NODE_BLAKE3><<<n_trees, 128, 0, side>>>(words, trees, run.result_dev);
+    SideFork fork(c, !c->capturing, 0);
+    if (kind == NODE_AES_MMO) bf_verify_batch_kernel<NODE_AES_MMO><<<n_trees, 128, 0, fork.side>>>(words, trees, run.result_dev);
+    else bf_verify_batch_kernel<NODE_BLAKE3><<<n_trees, 128, 0, fork.side>>>(words, trees, run.result_dev);
     ZKB_LAUNCHED(c);
-    bf_verify_chain_kernel<<<1, 32, exclusive_smem(bf_verify_chain_kernel, c), main_stream>>>(tr, words, log_n, point_dev, n_point, alpha, qidx);
+    bf_verify_chain_kernel<<<1, 32, exclusive_smem(bf_verify_chain_kernel, c), fork.main>>>(tr, words, log_n, point_dev, n_point, alpha, qidx);
     ZKB_LAUNCHED(c);
     const u32 items = log_n * BF_QUERIES;
-    bf_verify_fold_kernel<<<(items + 7) / 8, 256, 0, main_stream>>>(words, trees, log_n, alpha, qidx, tb.w_flat, run.result_dev + n_trees);
+    bf_verify_fold_kernel<<<(items + 7) / 8, 256, 0, fork.main>>>(words, trees, log_n, alpha, qidx, tb.w_flat, run.result_dev + n_trees);
     ZKB_LAUNCHED(c);
-    if (side != main_stream) {
-        cudaEvent_t join = c->side_event(1);
-        ZKB_CUDA(cudaEventRecord(join, side));
-        ZKB_CUDA(cudaStreamWaitEvent(main_stream, join, 0));
-    }
+    fork.join();
     ZKB_CUDA(cudaGetLastError());
     return run;
 }

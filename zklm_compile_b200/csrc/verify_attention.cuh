@@ -360,16 +360,11 @@ inline AvRun attention_verify_enqueue(zkb_ctx* c, TrState* tr, const AvParsed& p
     u64 n64 = L.S;
     memcpy(pre + 23, &n64, 8);
     const bool in_order = c->opt_bf_in_order || c->capturing || !tr;       // without a transcript to advance there is nothing to overlap
-    cudaStream_t rows_stream = in_order ? c->stream : c->side_stream();
-    if (!in_order) {
-        ZKB_CUDA(cudaEventRecord(c->side_event(0), c->stream));
-        ZKB_CUDA(cudaStreamWaitEvent(rows_stream, c->side_event(0), 0));
-    }
+    SideFork fork(c, !in_order, 0);
     AvArgs A{k, v, rec, bind, run.result_dev, att_heads_per_group(pr.num_heads, num_kv_heads), num_kv_heads != 0};
     const int threads = c->opt_att_threads ? c->opt_att_threads : ((L.s_pad >= 512 || L.d_pad > 128) ? 256 : 128);
-    attention_verify_kernel<<<run.rows, threads, smem, rows_stream>>>(A, L, b3_prefix(pre, 31));
+    attention_verify_kernel<<<run.rows, threads, smem, fork.side>>>(A, L, b3_prefix(pre, 31));
     ZKB_LAUNCHED(c);
-    if (!in_order) ZKB_CUDA(cudaEventRecord(c->side_event(1), rows_stream));
     if (tr) {
         ScriptBuilder sb;
         sb.word(pr.num_heads);
@@ -378,7 +373,7 @@ inline AvRun attention_verify_enqueue(zkb_ctx* c, TrState* tr, const AvParsed& p
         sb.words_dev(bind, (u32)pr.bind.size());
         sb.run(c, tr);
     }
-    if (!in_order) ZKB_CUDA(cudaStreamWaitEvent(c->stream, c->side_event(1), 0));
+    fork.join();
     ZKB_CUDA(cudaGetLastError());
     return run;
 }

@@ -232,25 +232,16 @@ inline BvRun basefold_batch_verify_enqueue(zkb_ctx* c, TrState* tr, const BbvPar
     ZKB_CUDA(cudaMemcpyAsync(add_first, pr.add_first.data(), (size_t)log_n * 4, cudaMemcpyHostToDevice, c->stream));
     ZKB_CUDA(cudaMemcpyAsync(add_count, pr.add_count.data(), (size_t)log_n * 4, cudaMemcpyHostToDevice, c->stream));
     ZKB_CUDA(cudaMemsetAsync(run.result_dev, 0, (size_t)run.n_results * 4, c->stream));
-    cudaStream_t main_stream = c->stream, side = c->capturing ? main_stream : c->side_stream();
-    if (side != main_stream) {
-        cudaEvent_t fork = c->side_event(0);
-        ZKB_CUDA(cudaEventRecord(fork, main_stream));
-        ZKB_CUDA(cudaStreamWaitEvent(side, fork, 0));
-    }
-    if (kind == NODE_AES_MMO) bf_verify_batch_kernel<NODE_AES_MMO><<<n_trees, 128, 0, side>>>(words, trees, run.result_dev);
-    else bf_verify_batch_kernel<NODE_BLAKE3><<<n_trees, 128, 0, side>>>(words, trees, run.result_dev);
+    SideFork fork(c, !c->capturing, 0);
+    if (kind == NODE_AES_MMO) bf_verify_batch_kernel<NODE_AES_MMO><<<n_trees, 128, 0, fork.side>>>(words, trees, run.result_dev);
+    else bf_verify_batch_kernel<NODE_BLAKE3><<<n_trees, 128, 0, fork.side>>>(words, trees, run.result_dev);
     ZKB_LAUNCHED(c);
-    bbv_chain_kernel<<<1, 32, exclusive_smem(bbv_chain_kernel, c), main_stream>>>(tr, words, pr.k, pr.roots_off, pr.batched_off, pr.fold_off, log_n, rho, alpha, qidx);
+    bbv_chain_kernel<<<1, 32, exclusive_smem(bbv_chain_kernel, c), fork.main>>>(tr, words, pr.k, pr.roots_off, pr.batched_off, pr.fold_off, log_n, rho, alpha, qidx);
     ZKB_LAUNCHED(c);
     const u32 items = log_n * BF_QUERIES;
-    bbv_fold_kernel<<<(items + 7) / 8, 256, 0, main_stream>>>(words, trees, log_n, rho, alpha, qidx, tb.w_flat, adds, add_first, add_count, run.result_dev + n_trees);
+    bbv_fold_kernel<<<(items + 7) / 8, 256, 0, fork.main>>>(words, trees, log_n, rho, alpha, qidx, tb.w_flat, adds, add_first, add_count, run.result_dev + n_trees);
     ZKB_LAUNCHED(c);
-    if (side != main_stream) {
-        cudaEvent_t join = c->side_event(1);
-        ZKB_CUDA(cudaEventRecord(join, side));
-        ZKB_CUDA(cudaStreamWaitEvent(main_stream, join, 0));
-    }
+    fork.join();
     ZKB_CUDA(cudaGetLastError());
     return run;
 }
