@@ -148,7 +148,9 @@ __device__ __forceinline__ u32 sha_madd(u32 a, u32 one, u32 b) { u32 r; asm("mad
         d = sha_madd(sha_madd(y_, one, ch_), one, s1_);                           \
         h = d + s0_ + md_;                                                        \
     }
-__device__ __noinline__ Sha8 sha256_rounds(Sha8 hin, const u32* __restrict__ kw) {
+// kw is shared memory that other lanes have just written and will write again: the loads below say that they read it ("memory"),
+// so no store is moved across them whatever the call is inlined into.
+__device__ __noinline__ Sha8 sha256_rounds(Sha8 hin, const u32* kw) {
     u32 one = SHA_ONE, minus_one = 0u - SHA_ONE;
     asm volatile("" : "+r"(one), "+r"(minus_one));
     const u32 kwa = (u32)__cvta_generic_to_shared(kw);
@@ -158,7 +160,7 @@ __device__ __noinline__ Sha8 sha256_rounds(Sha8 hin, const u32* __restrict__ kw)
         u32 k[8];
 #pragma unroll
         for (int j = 0; j < 8; j += 4)
-            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(k[j]), "=r"(k[j + 1]), "=r"(k[j + 2]), "=r"(k[j + 3]) : "r"(kwa + 4 * (i + j)));
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(k[j]), "=r"(k[j + 1]), "=r"(k[j + 2]), "=r"(k[j + 3]) : "r"(kwa + 4 * (i + j)) : "memory");
         ZKB_SHA_RND_KW(a, b, c, d, e, f, g, h, k[0]);
         ZKB_SHA_RND_KW(h, a, b, c, d, e, f, g, k[1]);
         ZKB_SHA_RND_KW(g, h, a, b, c, d, e, f, k[2]);
