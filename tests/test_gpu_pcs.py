@@ -106,6 +106,22 @@ def test_basefold_in_order_and_run_ahead_schedules_agree(ctx, kind):
             ctx.set_option(ctx.OPT_BASEFOLD_IN_ORDER, 0)
 
 
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("n_point,in_order", [(21, 1), (3, 0)])
+def test_basefold_rounds_that_share_buffers_at_the_size_of_subtrees_per_thread(ctx, kind, n_point, in_order):
+    """In order, and with a point of fewer coordinates than rounds (the later challenges are squeezed), two codewords and two trees
+    are written in turn: here with folds that take the kernel for levels of 2^20 inputs and more."""
+    n = (1 << 21) - 3
+    c, pt = rnd(43, n), rnd(44, n_point)
+    tg, to = zk.Transcript(ctx, b"bf-turn"), O.Transcript(b"bf-turn")
+    ctx.set_option(ctx.OPT_BASEFOLD_IN_ORDER, in_order)
+    try:
+        assert zp.basefold_commit_and_prove(ctx, tg, c, pt, kind) == O.basefold_commit_and_prove(to, c, pt, kind)
+    finally:
+        ctx.set_option(ctx.OPT_BASEFOLD_IN_ORDER, 0)
+    assert tg.squeeze() == to.squeeze()
+
+
 def _verify_both(ctx, blob, point, claimed, kind, label=b"bf-verify"):
     """(GPU decision, oracle decision); undecodable bytes are -1 on both sides."""
     to = O.Transcript(label)

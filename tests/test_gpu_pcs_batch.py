@@ -64,6 +64,17 @@ def test_ragged_batches(ctx, sizes, log_ns):
     b.close()
 
 
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("sizes,log_ns", [(((1 << 21) - 5, 1 << 20, (1 << 19) - 1), (21, 20, 19)), ((1 << 21, 1 << 19), (21, 19))])
+def test_joins_at_the_size_of_subtrees_per_thread(ctx, kind, sizes, log_ns):
+    """Folds of 2^20 values and more, which take the other tree kernel: with a polynomial that joins at the first fold (it is added to
+    the codeword's half as it stands) and at the second, and with none at the first (the half and its tree are used again)."""
+    rng = np.random.default_rng(sum(sizes))
+    b, got, exp, sg, so = both(ctx, [rng.integers(0, P, n).astype(np.uint32) for n in sizes], list(log_ns), False, kind)
+    assert got == exp and sg == so
+    b.close()
+
+
 def test_device_resident_polynomials_and_in_order_schedule(ctx):
     rng = np.random.default_rng(8)
     sizes, log_ns = (3000, 1000, 1024), [12, 10, 10]
