@@ -53,23 +53,39 @@ def schedule_bytes(n, launches, split=False):
     third time, folds r_0 and r_1 at once and writes the quarter-length EF tables (8 N + 8 N), and
     launch k >= 3 folds r_(k-1): reads two EF tables of N / 2^(k-1) elements and writes them at half
     length (96 N / 2^k).  In all 56 N per sumcheck against 72 N in the per-round formula above
-    (which has the first fold write half-length EF tables) and 80 N when round 0 is a separate pass."""
+    (which has the first fold write half-length EF tables).
+
+    Below 2^15 elements the two-challenge fold does not apply: launch 0 reads the base tables (8 N), launch 1 reads them
+    again, folds r_0 and writes half-length EF tables (8 N + 16 N), launch k >= 2 folds r_(k-1) (96 N / 2^k): 80 N."""
     N = 1 << n
-    if not split:
-        return ([8 * N, 16 * N] + [96 * N >> (k + 1) for k in range(2, launches)])[:launches]
-    per = [8 * N, 8 * N, 16 * N]
-    for k in range(3, launches):
-        per.append(96 * N >> k)
+    if n < 15:
+        per = [8 * N, 24 * N] + [96 * N >> k for k in range(2, launches)]
+    elif split:
+        per = [8 * N, 8 * N, 16 * N] + [96 * N >> k for k in range(3, launches)]
+    else:
+        per = [8 * N, 16 * N] + [96 * N >> (k + 1) for k in range(2, launches)]
     return per[:launches]
 
 
 def schedule_total(n, split=False):
-    return (56 if split else 48) << n
+    """The same over all launches, as a multiple of N: the launches' bytes and what the tail would move if it ran as launches."""
+    return 80 if n < 15 else (56 if split else 48)
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) over the schedule bytes above, from the ncu
-# captures summarised in profiles/sumcheck_kernels_product_ef.md (n = 25, one launch of each kernel of the split schedule).
-NCU_TRAFFIC_RATIO = {0: 1.02, 1: 1.02, 2: 0.92, "ef": 0.90}
+def schedule_kernels(n, split=False):
+    """Names of the first launches, and for each the DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) over the schedule
+    bytes above, from the ncu captures summarised in profiles/ (n = 25, one launch of each kernel; None: not captured)."""
+    if n < 15:
+        return [("sc_product_base_kernel<Fe,false> (round-0 message: reads both base tables)", None),
+                ("sc_product_base_kernel<Fe,true> (reads both base tables, folds r_0, writes half-length EF tables, round-1 message)", None)]
+    fold2 = ("sc_product_base_fold2_kernel (reads both base tables, folds r_0 and r_1, writes the quarter-length EF tables, round-2 message)", 0.92)
+    if split:
+        return [("sc_product_base_kernel<Fe,false> (round-0 message: reads both base tables)", 1.02),
+                ("sc_product_base_kernel<Fe,true,false> (round-1 message from nine coefficient sums: reads both base tables)", 1.02), fold2]
+    return [("sc_product_base_two_kernel (rounds 0 and 1 from nine coefficient sums: reads both base tables)", 1.01), fold2]
+
+
+EF_TRAFFIC_RATIO = 0.90     # sc_round_kernel over EF tables, as above
 
 
 def table_values(seed, first, count, step=1):
@@ -317,22 +333,17 @@ def sumcheck_roofline(n_local, prof, peak, src, world=1):
     sched = schedule_bytes(n_local, multi, split)
     rows = [(sched[i] / (prof[i] * 1e-3) / 1e9, prof[i], i) for i in range(multi) if prof[i] > 0]
     dom = max(rows, key=lambda t: t[1]) if rows else (0.0, 0.0, 0)
-    names = {0: "sc_product_base_kernel<Fe,false> (round-0 message: reads both base tables)",
-             1: "sc_product_base_kernel<Fe,true,false> (round-1 message from nine coefficient sums: reads both base tables)",
-             2: "sc_product_base_fold2_kernel (reads both base tables, folds r_0 and r_1, writes the quarter-length EF tables, round-2 message)"}
-    kname = names.get(dom[2], f"sc_round_kernel<PRODUCT,Fe,Fe,fold> (launch {dom[2]}: folds r_{dom[2] - 1}, round-{dom[2]} message)")
-    ratio = NCU_TRAFFIC_RATIO.get(dom[2] if dom[2] < 3 else "ef")
-    if not split:
-        kname = {0: "sc_product_base_two_kernel (rounds 0 and 1 from nine coefficient sums: reads both base tables)",
-                 1: names[2]}.get(dom[2], f"sc_round_kernel<PRODUCT,Fe,Fe,fold> (launch {dom[2]}: folds r_{dom[2]}, round-{dom[2] + 1} message)")
-        ratio = None
+    first = schedule_kernels(n_local, split)
+    last_folded = dom[2] if not split and n_local >= 15 else dom[2] - 1     # the newest challenge that an EF launch folds in
+    kname, ratio = first[dom[2]] if dom[2] < len(first) else (f"sc_round_kernel<PRODUCT,Fe,Fe,fold> (launch {dom[2]}: folds r_{last_folded}, "
+                                                              f"round-{last_folded + 1} message)", EF_TRAFFIC_RATIO if n_local >= 15 else None)
     l2 = 126e6
     big = [r for r in rows if sched[r[2]] > 2 * l2]
     return {"bound": "hbm", "achieved": round(dom[0], 1), "peak": peak, "unit": "GB/s", "frac": round(dom[0] / peak, 4) if peak else None,
             "traffic": int(ratio * sched[dom[2]]) if ratio else None,
             "traffic_source": "bytes of the launch x the dram/bytes ratio ncu measured on this kernel at n = 25 (profiles/)" if ratio else None,
             "peak_source": src, "kernel": f"{kname}: {sched[dom[2]]} bytes in {dom[1]:.4f} ms" + (f" on one of {world} GPUs" if world > 1 else ""),
-            "bytes_definition": f"bytes the launch must move in this schedule; the whole sumcheck moves {56 if split else 48} * 2^n "
+            "bytes_definition": f"bytes the launch must move in this schedule; the whole sumcheck moves {schedule_total(n_local, split)} * 2^n "
                                 "bytes where the per-round formula of the metric counts 72 * 2^n",
             "per_launch_gbps": [round(t[0], 1) for t in rows[:14]], "per_launch_ms": [round(t, 4) for t in prof[:16]],
             "per_launch_frac": [round(t[0] / peak, 3) for t in rows[:14]] if peak else None,
@@ -373,8 +384,8 @@ def run_sumcheck(zk, ctx, n, steps, warmup, rank, with_e2e, barrier=lambda: None
     res = {"n": n, "value_gbps": round(world * total_bytes / (ms_step * 1e-3) / 1e9, 2), "ms_per_step": round(ms_step, 4),
            "proof_sha256": hashlib.sha256(out[0].round_polys.tobytes() + out[0].challenges.tobytes()).hexdigest(),
            "frac_of_peak_whole_sumcheck": round(total_bytes / (ms_step * 1e-3) / 1e9 / peak, 4),
-           "value_by_schedule_bytes_gbps": round(world * schedule_total(n) / (ms_step * 1e-3) / 1e9, 2),
-           "gpu_launches": int(launches), "algorithmic_bytes_per_step": total_bytes, "schedule_bytes_per_step": schedule_total(n),
+           "value_by_schedule_bytes_gbps": round(world * schedule_total(n) * N / (ms_step * 1e-3) / 1e9, 2),
+           "gpu_launches": int(launches), "algorithmic_bytes_per_step": total_bytes, "schedule_bytes_per_step": schedule_total(n) * N,
            "roofline": sumcheck_roofline(n, prof, peak, src)}
     if with_e2e:
         for _ in range(2):

@@ -1,4 +1,4 @@
-"""Host-side pieces of bench.py that need no GPU: the clock sampler's windowing."""
+"""Host-side pieces of bench.py that need no GPU: the clock sampler's windowing and the byte counts of the sumcheck's launches."""
 import importlib.util
 import os
 
@@ -44,3 +44,17 @@ def test_clock_sampler_falls_back_to_all_samples_and_reports_reasons():
 def test_clock_sampler_without_nvidia_smi():
     s = bench.ClockSampler(0)
     assert s.stop()["reasons"] == ["nvidia-smi unavailable"]
+
+
+def test_launch_bytes_add_up_to_the_schedule_of_each_form():
+    for n, split, words in ((28, False, 48), (28, True, 56), (15, False, 48), (14, False, 80)):
+        per = bench.schedule_bytes(n, n + 2, split)
+        assert bench.schedule_total(n, split) == words
+        assert words - 1 < sum(per) / (1 << n) <= words           # the last rounds are what is left of the geometric sum
+        named = bench.schedule_kernels(n, split)
+        prof = [1.0] * 5
+        for i in range(4):
+            prof[i] = 9.0
+            r = bench.sumcheck_roofline(n, prof, 6434.8, "t", 2 if split else 1)
+            prof[i] = 1.0
+            assert r["kernel"].startswith(named[i][0] if i < len(named) else "sc_round_kernel") and f": {per[i]} bytes" in r["kernel"]
