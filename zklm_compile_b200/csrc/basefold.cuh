@@ -364,9 +364,12 @@ inline void mk_launch(zkb_ctx* c, int mode, const u32* values, size_t n_valid, s
     }
     const size_t tile = n_in < (size_t)MK_TILE ? n_in : (size_t)MK_TILE;
     const unsigned grid = (unsigned)(n_in / tile);
-    if (mode == MK_VALUES) mk_tile_kernel<KIND, MK_VALUES><<<grid, MK_THREADS, 0, c->stream>>>(values, n_valid, n_in, k0, h, nodes, f);
-    else if (mode == MK_DIGESTS) mk_tile_kernel<KIND, MK_DIGESTS><<<grid, MK_THREADS, 0, c->stream>>>(values, n_valid, n_in, k0, h, nodes, f);
-    else mk_tile_kernel<KIND, MK_FOLD><<<grid, MK_THREADS, 0, c->stream>>>(values, n_valid, n_in, k0, h, nodes, f);
+    const bool doubled = f.doubled && grid == 1;
+    if (mode == MK_VALUES && doubled) mk_tile_kernel<KIND, MK_VALUES, true><<<grid, MK_THREADS, 0, c->stream>>>(values, n_valid, n_in, k0, h, nodes, f);
+    else if (mode == MK_VALUES) mk_tile_kernel<KIND, MK_VALUES, false><<<grid, MK_THREADS, 0, c->stream>>>(values, n_valid, n_in, k0, h, nodes, f);
+    else if (mode == MK_DIGESTS && doubled) mk_tile_kernel<KIND, MK_DIGESTS, true><<<grid, MK_THREADS, 0, c->stream>>>(values, n_valid, n_in, k0, h, nodes, f);
+    else if (mode == MK_DIGESTS) mk_tile_kernel<KIND, MK_DIGESTS, false><<<grid, MK_THREADS, 0, c->stream>>>(values, n_valid, n_in, k0, h, nodes, f);
+    else mk_tile_kernel<KIND, MK_FOLD, false><<<grid, MK_THREADS, 0, c->stream>>>(values, n_valid, n_in, k0, h, nodes, f);
     ZKB_LAUNCHED(c);
 }
 // Build every layer of a tree of height h; the first launch reads leaves (values, or a fold).
