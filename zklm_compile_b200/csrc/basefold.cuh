@@ -133,8 +133,9 @@ __device__ __forceinline__ void bf_butterflies(u32* e, const u32* tw) {
 // Levels 0..11 on tiles of 2^12 coefficients, four levels at a time on sixteen values in a thread's registers: three trips
 // through shared memory instead of twelve, and fifteen factors for 32 butterflies.  One word of padding per sixteen keeps
 // the strided accesses on different banks.
-// Bound by shared-memory and integer issue, not by HBM.  Measured on B200 with a level at a time in shared memory -> with this
-// and the high levels three at a time: a whole opening of 2^24 coefficients 3053 -> 2929 us.
+// Bound by integer issue behind the loads of coefficients and factors (ncu at 2^22: ALU pipe 55 %, shared memory 17 %, DRAM 6 %).  Measured
+// on B200 with a level at a time in shared memory -> with this and the high levels three at a time: a whole opening of 2^24
+// coefficients 3053 -> 2929 us, encoding both halves of them 389 -> 259 us.
 __global__ void __launch_bounds__(256) bf_encode_low12_kernel(CoefSrc src, const u32* __restrict__ t_flat, u32* __restrict__ cw, size_t n_pad, int dup) {
     __shared__ u32 sm[(1 << BF_LOW_LOG) + (1 << (BF_LOW_LOG - 4))];
     const size_t base = (size_t)blockIdx.x << BF_LOW_LOG;
@@ -241,7 +242,7 @@ __device__ __forceinline__ u32 bf_next_alpha(Tr& tr, const u32* point, u32 n_poi
     return tr_squeeze(tr);
 }
 // The transcript's part of some rounds: absorb the folded root, squeeze the query positions, take the next challenge.  This
-// is the opening's critical path (26 dependent SHA-256 compressions a round, one thread, about 58 us), so nothing else is in
+// is the opening's critical path (26 dependent SHA-256 compressions a round on one thread: 46 us, 1.77 us each), so nothing else is in
 // it: the paths are gathered by bf_gather_kernel, off the chain.  Measured on B200 with the gathers inside and a launch per
 // round -> like this: Basefold of 2^24 coefficients 3213 -> 3053 us.
 __global__ void __launch_bounds__(32) bf_chain_kernel(const __grid_constant__ BfRounds a) {
@@ -419,8 +420,9 @@ inline void bf_launch_chain(zkb_ctx* c, const BfRounds& a) {
 }
 // How many rounds the chain launch that starts at `round` takes when the trees run ahead on another stream: one while the
 // folded codewords are long (the next tree is still being built when this round's positions are known), then four,
-// then all the rest, whose small trees are finished long before the chain gets to them (58 us a round at the slowest,
-// about 13 us a tree).
+// then all the rest.  The line is where a fold and its tree take less than the chain's 46 us a round, so that from there on the
+// trees run away from the chain; measured on B200 alone on one stream, blake3 / AES: 2^20 values 71 / 82 us, 2^19 51 / 67, 2^18 37 / 48,
+// 2^17 29 / 39, 2^15 27 / 37, 2^10 16 / 24.
 inline u32 bf_chain_rounds(u32 round, u32 log_n) {
     const u32 long_rounds = log_n > 18 ? log_n - 18 : 0;
     const u32 n = round < long_rounds ? 1 : (round == long_rounds ? 4 : log_n);

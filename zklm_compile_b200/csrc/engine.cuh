@@ -63,8 +63,9 @@ inline int grid_for(zkb_ctx* c, size_t items, int per_cta = 256, int ctas_per_sm
 
 
 // fused2: product sumcheck over base tables with EF challenges whose destination tables were sized
-// for the two-challenge fold (a quarter of the input): round 1 is a message-only launch and the
-// first tables written are those folded with r_0 and r_1 (sc_product_base_fold2_kernel).
+// for the two-challenge fold (a quarter of the input): the first tables written are those folded with r_0 and r_1
+// (sc_product_base_fold2_kernel).  On one GPU rounds 0 and 1 share a message-only launch in front of it; split over
+// several GPUs each has its own, since their sums are exchanged round by round.
 template <int KIND, class SrcT, class ChalT>
 void run_sumcheck(zkb_ctx* c, ScTables tb, u32 num_vars, ScIO io, bool dynamic, bool fused2 = false) {
     // split over several GPUs: the tables are this GPU's slice of 2^local_vars elements

@@ -248,10 +248,11 @@ __global__ void __launch_bounds__(MK_THREADS) mk_tile_kernel(const u32* __restri
 // fifteen nodes one after the other in post-order, the nodes that wait for their sibling in registers.  No lane is ever
 // idle and no barrier separates the levels; in a tile the last five levels run on part of a warp, and most warps wait.
 // Leaves are staged (and folded) through shared memory with coalesced accesses, one word of padding per thread.
-// Bound by integer issue; the tile kernel reached 26.9 G blake3 nodes/s against 37 for the node alone.  Measured on B200
-// with the tile kernel -> with this one at the top: Basefold of 2^24 coefficients 3475 -> 3213 us (blake3), a batch of seven
-// polynomials up to 2^22 2682 -> 2452 us (AES).  Below 2^20 inputs there are fewer than 2^16 subtrees, not four warps to a
-// scheduler, and fifteen nodes in a row would take longer than a tile's ten levels.
+// Bound by integer issue (ncu: ALU pipe 90 % busy, DRAM 3 %): 34.6 G blake3 nodes/s over 2^24 leaves, 33.2 G AES nodes/s, where the
+// tile kernel reached 26.9 G blake3 nodes/s and the node alone runs at 37.  Measured on B200 with the tile kernel -> with this
+// one at the top: Basefold of 2^24 coefficients 3475 -> 3213 us (blake3), a batch of seven polynomials up to 2^22 2682 -> 2452 us
+// (AES).  Below 2^20 inputs there are fewer than 2^16 subtrees, not four warps to a scheduler, and fifteen nodes in a row would
+// take longer than a tile's ten levels.
 constexpr int MK_LANE_LOG = 4, MK_LANE = 1 << MK_LANE_LOG, MK_LANE_THREADS = 256;
 constexpr size_t mk_lane_smem(int kind) { return kind == NODE_AES_MMO ? AES_REP_WORDS * 4 : 0; }
 constexpr size_t MK_LANE_MIN = size_t(1) << 20;      // inputs: below, the subtrees are too few to fill the GPU

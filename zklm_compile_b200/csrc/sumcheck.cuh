@@ -255,8 +255,7 @@ __device__ __forceinline__ void ld4(const void* base, size_t j, u32* o) {
     o[0] = t.x; o[1] = t.y; o[2] = t.z; o[3] = t.w;
 }
 
-// WRITE = false (with FOLD): the folded tables are not materialised - the launch only produces
-// the round message (the fused launch below folds two challenges at once from the base tables).
+// The nine coefficient sums of one pair index: quarters (a, b, c, d) of f and g.
 __device__ __forceinline__ void sc_base_coef_accum(u64* acc, u32 fa, u32 fb, u32 fc, u32 fd, u32 ga, u32 gb, u32 gc, u32 gd) {
     const u32 ef = sub31(fb, fa), eg = sub31(gb, ga);       // lo = a + r e
     const u32 hf = sub31(fd, fc), hg = sub31(gd, gc);       // hi = c + r h
@@ -272,6 +271,8 @@ __device__ __forceinline__ void sc_base_coef_accum(u64* acc, u32 fa, u32 fb, u32
     acc[7] += fold62((u64)pf * qg + (u64)pg * qf);
     acc[8] += fold62((u64)qf * qg);
 }
+// WRITE = false (with FOLD): the folded tables are not materialised - the launch only produces
+// the round message (the fused launch below folds two challenges at once from the base tables).
 template <class ChalT, bool FOLD, bool WRITE = true>
 __global__ void __launch_bounds__(256) sc_product_base_kernel(ScTables tb, size_t half, u32 round, ScIO io) {
     constexpr int NACC = FOLD ? 9 : 3;
@@ -457,10 +458,10 @@ __global__ void __launch_bounds__(256) sc_product_base_fold2_kernel(ScTables tb,
 // The nine coefficient sums of round 1 determine round 0 as well: with quarters (a, b, c, d) of the tables, s(0) = sum (a a +
 // c c) = A0 + C0, s(1) is both quadratics at r = 1 and s(2) both at r = 2.  So one pass over the tables serves both
 // rounds: the finishing CTA hashes the first message, evaluates the quadratics at the challenge and hashes the second.  The
-// launch is bound by HBM (it reads 8 N bytes, N elements to a table); a launch for each round read them twice.
-// Measured on B200 at n = 28, a launch for each round -> this one: 3425 -> 3119 us for the whole sumcheck.
+// launch is bound by HBM (it reads 8 N bytes, N elements to a table: 0.40 ms at n = 28, 5.3 TB/s); a launch for each round read them
+// twice (0.35 + 0.34 ms).  Measured on B200 at n = 28, a launch for each round -> this one: 3425 -> 3119 us for the whole sumcheck.
 // (Two rounds per launch on the extension-field tables behind it move 37 N bytes in all instead of 48 N, but there
-// a pair costs nine EF products, about 2600 issue slots of field reductions with the folds: bound by those, not kept.)
+// a pair costs nine EF products, about 2600 issue slots of field reductions with the folds: 3292 us, not kept.)
 // `q` = a quarter of the tables' length, a multiple of four.
 __global__ void __launch_bounds__(256) sc_product_base_two_kernel(ScTables tb, size_t q, u32 round, ScIO io) {
     __shared__ u32 red[32 * 16];

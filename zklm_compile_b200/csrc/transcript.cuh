@@ -61,7 +61,7 @@ __device__ __forceinline__ u32 bswap32(u32 x) { return __byte_perm(x, 0, 0x0123)
 // strict dependency chain, so the remaining lever is instruction count, not parallelism.
 struct Sha8 { u32 v[8]; };
 
-// One round.  A lone warp issues an integer instruction about every two cycles (measured on B200:
+// One round.  The logic and shift pipe takes an instruction of a lone warp about every two cycles (measured on B200:
 // eight independent lop3 or shf per iteration run at 2.0 - 2.2 cycles each, a dependent one at 4.4),
 // so a compression is bound by its instruction count, not by the dependency chain: the boolean
 // functions are single lop3 instructions, and the additions are written as multiply-adds by one in
@@ -131,9 +131,12 @@ __device__ __noinline__ Sha8 sha256_compress(Sha8 hin, const u32* __restrict__ b
 // compiler cannot see through (it turns a multiply by a literal one back into an add).  Ten of the logic pipe's slots are
 // fixed (six rotations, four lop3); of the additions only the three-operand one of a' stays there, in the form
 // e' = h + kw + d + ch + s1,  a' = e' + s0 + (maj - d).  With the schedule words read sixteen bytes at a time.
-// Measured on B200: a lone lane's 64 rounds 1955 cycles in the form of ZKB_SHA_RND, 1763 in this one (both with words read one
-// by one); checking 1232 attention rows with the caller's transcript of 15 800 blocks 18.9 -> 15.2 ms.  Inside a whole
-// compression, where the schedule's additions compete for the same pipes, this form is slower than ZKB_SHA_RND.
+// Measured on B200: a lone lane's 64 rounds, unrolled, 1915 cycles in the form of ZKB_SHA_RND and 1763 in this one (both with words
+// read one by one; ZKB_SHA_RND rolled by sixteen 1955); checking 1232 attention rows with the caller's transcript of 15 800 blocks
+// 19.2 -> 15.0 ms, 0.87 us a block.  Inside a whole compression, where the schedule's additions compete for the same pipes, this
+// form is slower than ZKB_SHA_RND.
+// Unrolled over the block.  The same rolled by sixteen rounds, rolled -> unrolled: that check 15.9 -> 15.0 ms, the GPT-2 shape 53.1 ->
+// 52.6, four 4B-shape layers no difference, thirty-two side by side on one GPU 25.0 -> 25.6 (25.9 before this form).
 constexpr int SHA_KW_STRIDE = 68;    // whole 16-byte vectors; lanes that write their own row stay on different banks
 __constant__ u32 SHA_ONE = 1u;
 __device__ __forceinline__ u32 sha_madd(u32 a, u32 one, u32 b) { u32 r; asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(one), "r"(b)); return r; }
@@ -420,7 +423,7 @@ __device__ __forceinline__ void tr_absorb_stream_warp(Tr& tr, u32 total, Load lo
 }
 
 // The same absorb for a CTA of two warps with the loads and the schedule expansion taken off the
-// hash chain: while lane 0 of warp 0 runs the rounds of one batch (up to 32 blocks, about 35 us),
+// hash chain: while lane 0 of warp 0 runs the rounds of one batch (up to 32 blocks, about 28 us),
 // warp 1 fetches the next batch's words and expands its schedules into the other half of the
 // double-buffered scratch; the two meet at a CTA barrier per batch.  Called by all 64 threads with
 // identical arguments; `tr` is meaningful in thread 0; `bufw` is the stream buffer (shared
