@@ -34,26 +34,32 @@ __global__ void __launch_bounds__(256) bfb_lincomb_kernel(const u32* const* __re
     }
 }
 // Absorb the batched root, squeeze the whole fold point, absorb its first coordinate (:1277-1291).
-__global__ void bfb_begin_kernel(TrState* st, const uint4* root, u32 log_n, u32* fold_point, u32* rec_root) {
+__global__ void __launch_bounds__(64) bfb_begin_kernel(TrState* st, const uint4* root, u32 log_n, u32* fold_point, u32* rec_root) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
-    Tr tr;
+    if (threadIdx.x >= 32) { tr_pair_help(trbuf); return; }
+    const bool lead = threadIdx.x == 0;
+    TrPair tr;
     tr_load(tr, st, trbuf);
     uint4 r = *root;
     u32 rw[4] = {r.x, r.y, r.z, r.w};
     tr_absorb_words<4>(tr, rw);
-    rec_root[0] = r.x; rec_root[1] = r.y; rec_root[2] = r.z; rec_root[3] = r.w;
-    for (u32 b = 0; b < log_n; b++) fold_point[b] = tr_squeeze(tr);
-    tr_absorb_u32(tr, fold_point[0]);
-    tr_store(tr, st);
+    if (lead) { rec_root[0] = r.x; rec_root[1] = r.y; rec_root[2] = r.z; rec_root[3] = r.w; }
+    u32 first = 0;
+    tr_squeeze_run(tr, log_n, [&](u32 b, u32 v) { if (b == 0) first = v; if (lead) fold_point[b] = v; });
+    tr_absorb_u32(tr, first);
+    tr_pair_end(tr);
+    if (lead) tr_store(tr, st);
 }
 // derive_query_indices(transcript, max_log_n + 1) after the last round (:1366), reduced mod 2^max_log_n as the
 // individual openings use them (:917-923).
-__global__ void bfb_final_kernel(TrState* st, u32 mask, u32* idx) {
+__global__ void __launch_bounds__(64) bfb_final_kernel(TrState* st, u32 mask, u32* idx) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
-    Tr tr;
+    if (threadIdx.x >= 32) { tr_pair_help(trbuf); return; }
+    TrPair tr;
     tr_load(tr, st, trbuf);
-    for (u32 q = 0; q < BF_QUERIES; q++) idx[q] = tr_squeeze(tr) & mask;
-    tr_store(tr, st);
+    tr_squeeze_run(tr, BF_QUERIES, [=](u32 q, u32 v) { if (threadIdx.x == 0) idx[q] = v & mask; });
+    tr_pair_end(tr);
+    if (threadIdx.x == 0) tr_store(tr, st);
 }
 // 48 raw paths of an individual tree: positions (idx[q] mod tree_half) and that + tree_half (:1330-1340, :917-927).
 __global__ void __launch_bounds__(256) bfb_open_kernel(const u32* __restrict__ values, const uint4* __restrict__ nodes, u32 h, const u32* __restrict__ idx,
@@ -135,7 +141,7 @@ BfbPending bfb_enqueue(zkb_bf_batch* B, TrState* tr, bool individual) {
     mk_build(c, kind, MK_VALUES, cw0, cw_len0, log_n, tree0, none);
     u32* fold_point = (u32*)c->scratch(((size_t)log_n + 1) * 4);
     pd.batched_root_off = c->rec_alloc(4);
-    bfb_begin_kernel<<<1, 1, 0, c->stream>>>(tr, tree0 + mk_node_count(log_n), log_n, fold_point, c->rec_dev + pd.batched_root_off);
+    bfb_begin_kernel<<<1, 64, 0, c->stream>>>(tr, tree0 + mk_node_count(log_n), log_n, fold_point, c->rec_dev + pd.batched_root_off);
     ZKB_LAUNCHED(c);
 
     const bool in_order = c->opt_bf_in_order || c->capturing;
@@ -215,7 +221,7 @@ BfbPending bfb_enqueue(zkb_bf_batch* B, TrState* tr, bool individual) {
         ZKB_LAUNCHED(c);
     }
     pd.final_idx_off = c->rec_alloc(BF_QUERIES);
-    bfb_final_kernel<<<1, 1, 0, c->stream>>>(tr, (u32(1) << log_n) - 1, c->rec_dev + pd.final_idx_off);
+    bfb_final_kernel<<<1, 64, 0, c->stream>>>(tr, (u32(1) << log_n) - 1, c->rec_dev + pd.final_idx_off);
     ZKB_LAUNCHED(c);
     if (individual) {
         for (u32 i = 0; i < k; i++) {

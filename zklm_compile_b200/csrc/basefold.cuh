@@ -237,18 +237,20 @@ __host__ __device__ __forceinline__ size_t bf_round_words(u32 h_prev) {
 }
 // The challenge of a round: the point coordinate (absorbed) while there is one, else a squeeze
 // (basefold.rs:508-513).
-__device__ __forceinline__ u32 bf_next_alpha(Tr& tr, const u32* point, u32 n_point, u32 round) {
+template <class T>
+__device__ __forceinline__ u32 bf_next_alpha(T& tr, const u32* point, u32 n_point, u32 round) {
     if (round < n_point) { u32 a = point[round]; tr_absorb_u32(tr, a); return a; }
     return tr_squeeze(tr);
 }
 // The transcript's part of some rounds: absorb the folded root, squeeze the query positions, take the next challenge.  This
-// is the opening's critical path (26 dependent SHA-256 compressions a round on one thread: 46 us, 1.77 us each), so nothing else is in
+// is the opening's critical path (26 dependent SHA-256 compressions a round), so nothing else is in
 // it: the paths are gathered by bf_gather_kernel, off the chain.  Measured on B200 with the gathers inside and a launch per
 // round -> like this: Basefold of 2^24 coefficients 3213 -> 3053 us.
-__global__ void __launch_bounds__(32) bf_chain_kernel(const __grid_constant__ BfRounds a) {
+__global__ void __launch_bounds__(64) bf_chain_kernel(const __grid_constant__ BfRounds a) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
-    if (threadIdx.x) return;
-    Tr tr;
+    if (threadIdx.x >= 32) { tr_pair_help(trbuf); return; }
+    const bool lead = threadIdx.x == 0;
+    TrPair tr;
     tr_load(tr, a.tr, trbuf);
     for (u32 round = a.first; round < a.first + a.count; round++) {
         const BfRound& p = a.r[round];
@@ -256,12 +258,17 @@ __global__ void __launch_bounds__(32) bf_chain_kernel(const __grid_constant__ Bf
         const uint4 root = p.fold_nodes[mk_layer_offset(h_fold, h_fold)];
         u32 rw[4] = {root.x, root.y, root.z, root.w};
         tr_absorb_words<4>(tr, rw);
-        p.rec[0] = root.x; p.rec[1] = root.y; p.rec[2] = root.z; p.rec[3] = root.w;
+        u32* rec = p.rec;
+        if (lead) { rec[0] = root.x; rec[1] = root.y; rec[2] = root.z; rec[3] = root.w; }
         const u32 prev_half_mask = (1u << (p.h_prev - 1)) - 1;
-        for (u32 q = 0; q < BF_QUERIES; q++) p.rec[4 + q] = tr_squeeze(tr) & prev_half_mask;     // (squeeze mod 2^h_prev) mod prev_half
-        if (p.alpha_next) *p.alpha_next = bf_next_alpha(tr, a.point, a.n_point, round + 1);
+        tr_squeeze_run(tr, BF_QUERIES, [=](u32 q, u32 v) { if (lead) rec[4 + q] = v & prev_half_mask; });     // (squeeze mod 2^h_prev) mod prev_half
+        if (p.alpha_next) {
+            const u32 v = bf_next_alpha(tr, a.point, a.n_point, round + 1);
+            if (lead) *p.alpha_next = v;
+        }
     }
-    tr_store(tr, a.tr);
+    tr_pair_end(tr);
+    if (lead) tr_store(tr, a.tr);
 }
 // The opened paths of those rounds, one warp each: blockIdx.y is the round, 3 * BF_QUERIES paths to a round.
 constexpr u32 BF_GATHER_WARPS = 8;
@@ -415,7 +422,7 @@ inline void bf_launch_gather(zkb_ctx* c, const BfRounds& a) {
     ZKB_LAUNCHED(c);
 }
 inline void bf_launch_chain(zkb_ctx* c, const BfRounds& a) {
-    bf_chain_kernel<<<1, 32, exclusive_smem(bf_chain_kernel, c), c->stream>>>(a);
+    bf_chain_kernel<<<1, 64, exclusive_smem(bf_chain_kernel, c), c->stream>>>(a);
     ZKB_LAUNCHED(c);
 }
 // How many rounds the chain launch that starts at `round` takes when the trees run ahead on another stream: one while the

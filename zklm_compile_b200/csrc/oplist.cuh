@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(TRSCRIPT_THREADS) hash_values_kernel(const u32
     __shared__ u32 bc[1];
     Tr tr;
     tr.buf = trbuf; tr.buflen = 0; tr.total = 0;
-    if (threadIdx.x == 0) { tr_iv(tr.h); tr_absorb_u32(tr, n); }
+    if (threadIdx.x < 32) { tr_iv(tr.h); tr_absorb_u32(tr, n); }
     tr_absorb_stream_2w(tr, n, [=](u32 g) -> u32 { return v[g]; }, reinterpret_cast<u32*>(trbuf), tile, kw, bc);
     if (threadIdx.x == 0) {
         u32 d[8];
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(TRSCRIPT_THREADS) hash_values_multi_kernel(con
     const u32 n = jobs[blockIdx.x].n;
     Tr tr;
     tr.buf = trbuf; tr.buflen = 0; tr.total = 0;
-    if (threadIdx.x == 0) { tr_iv(tr.h); tr_absorb_u32(tr, n); }
+    if (threadIdx.x < 32) { tr_iv(tr.h); tr_absorb_u32(tr, n); }
     tr_absorb_stream_2w(tr, n, [=](u32 g) -> u32 { return v[g]; }, reinterpret_cast<u32*>(trbuf), tile, kw, bc);
     if (threadIdx.x == 0) {
         u32 d[8];

@@ -68,10 +68,14 @@ __global__ void __launch_bounds__(1024) seq1_consistency_kernel(TrState* st, con
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     __shared__ Fp r_s[32], rv_s[32];
     __shared__ u32 red[64];
-    Tr tr;
-    if (threadIdx.x == 0) {
+    TrPair tr;
+    if (threadIdx.x < 32) {
         tr_load(tr, st, trbuf);
-        for (u32 i = 0; i < log_attn; i++) r_s[i].v = tr_squeeze(tr);
+        tr_squeeze_run(tr, log_attn, [&](u32 i, u32 v) { r_s[i].v = v; });
+        tr_pair_end(tr);
+    } else if (threadIdx.x < 64) tr_pair_help(trbuf);
+    __syncthreads();
+    if (threadIdx.x == 0) {
         if (!is_gqa) for (u32 i = 0; i < log_v; i++) rv_s[i] = r_s[i];
         else {
             for (u32 i = 0; i < log_kv; i++) rv_s[i] = r_s[i];
@@ -85,9 +89,12 @@ __global__ void __launch_bounds__(1024) seq1_consistency_kernel(TrState* st, con
     for (u32 i = threadIdx.x; i < v_len; i += blockDim.x)
         acc[1] = add31(acc[1], mul31(eq_at_index<Fp>(rv_s, log_v, i).v, v[i]));
     block_sum_words<2>(acc, red);
+    if (threadIdx.x < 32) {
+        TrWarp& alone = tr;                   // one compression at most
+#pragma unroll
+        for (int k = 0; k < 2; k++) tr_absorb_u32(alone, __shfl_sync(0xffffffffu, acc[k], 0));
+    }
     if (threadIdx.x == 0) {
-        tr_absorb_u32(tr, acc[0]);
-        tr_absorb_u32(tr, acc[1]);
         tr_store(tr, st);
         out2[0] = acc[0];
         out2[1] = acc[1];

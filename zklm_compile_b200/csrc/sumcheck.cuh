@@ -160,10 +160,10 @@ __device__ __forceinline__ void block_sum_words(u32* v, u32* red /* [32][NWORDS]
     __syncthreads();
 }
 
-// Thread 0: turn the summed accumulators into the round message, advance the transcript,
+// Warp 0, all lanes with the same words: turn the summed accumulators into the round message, advance the transcript,
 // emit the stored evaluations and the challenge.
-template <int KIND, class AccT, class ChalT>
-__device__ __forceinline__ ChalT sc_finish_round(const u32* words, const ScIO& io, u32 round, Tr& tr) {
+template <int KIND, class AccT, class ChalT, class T>
+__device__ __forceinline__ ChalT sc_finish_round(const u32* words, const ScIO& io, u32 round, T& tr) {
     constexpr int NACC = ScTraits<KIND>::NACC, NABS = ScTraits<KIND>::NABS;
     constexpr int WA = Width<AccT>::W, WC = Width<ChalT>::W;
     ChalT s[4];
@@ -174,18 +174,39 @@ __device__ __forceinline__ ChalT sc_finish_round(const u32* words, const ScIO& i
         widen_to(a, s[k]);
     }
     if constexpr (KIND == SC_ONES) s[2] = s[1] + s[1] - s[0];
-    if (io.check_zero_sum && round == 0 && !is_zero_el(s[0] + s[1])) atomicExch(io.status, 3u);
+    const bool lead = (threadIdx.x & 31) == 0;
+    if (lead && io.check_zero_sum && round == 0 && !is_zero_el(s[0] + s[1])) atomicExch(io.status, 3u);
     u32* out = io.polys + (size_t)round * NABS * WC;
     u32 msg[NABS * WC];
 #pragma unroll
     for (int k = 0; k < NABS; k++) to_words(s[k], msg + k * WC);
     tr_absorb_words<NABS * WC>(tr, msg);
+    if (lead) {
 #pragma unroll
-    for (int k = 0; k < NABS * WC; k++) out[k] = msg[k];
+        for (int k = 0; k < NABS * WC; k++) out[k] = msg[k];
+    }
     ChalT r;
     tr_squeeze_el(tr, r);
-    to_words(r, io.chal + (size_t)round * WC);
+    if (lead) to_words(r, io.chal + (size_t)round * WC);
     return r;
+}
+// The CTA that finished a round, with the NW sums in lane 0 of warp 0: warp 0 runs `hash` with the sums in every lane, its
+// compressions shared with warp 1.
+template <int NW, class Hash>
+__device__ __forceinline__ void sc_hash_by_pair(u32* t, const ScIO& io, unsigned char* trbuf, Hash hash) {
+    const int warp = threadIdx.x >> 5;
+    if (warp == 0) {
+#pragma unroll
+        for (int k = 0; k < NW; k++) t[k] = __shfl_sync(0xffffffffu, t[k], 0);
+        TrPair tr;
+        tr_load(tr, io.tr, trbuf);
+        hash(tr);
+        tr_pair_end(tr);
+        if (threadIdx.x == 0) {
+            tr_store(tr, io.tr);
+            *io.counter = 0;
+        }
+    } else if (warp == 1) tr_pair_help(trbuf);
 }
 
 // ---- multi-CTA round launch ----------------------------------------------------------------
@@ -230,13 +251,7 @@ __global__ void __launch_bounds__(256) sc_round_kernel(ScTables tb, size_t half,
     }
     block_sum_words<NW>(t, red);
     if (io.xch && threadIdx.x < 32) xch_allreduce_warp<NW>(*io.xch, io.xch->seq + round, t);
-    if (threadIdx.x == 0) {
-        Tr tr;
-        tr_load(tr, io.tr, trbuf);
-        sc_finish_round<KIND, AccT, ChalT>(t, io, round, tr);
-        tr_store(tr, io.tr);
-        *io.counter = 0;
-    }
+    sc_hash_by_pair<NW>(t, io, trbuf, [&](TrPair& tr) { sc_finish_round<KIND, AccT, ChalT>(t, io, round, tr); });
 }
 
 // ---- product sumcheck over base-field tables: the two bandwidth-critical launches --------------
@@ -341,9 +356,7 @@ __global__ void __launch_bounds__(256) sc_product_base_kernel(ScTables tb, size_
     }
     block_sum_words<NACC>(t, red);
     if (io.xch && threadIdx.x < 32) xch_allreduce_warp<NACC>(*io.xch, io.xch->seq + round, t);
-    if (threadIdx.x == 0) {
-        Tr tr;
-        tr_load(tr, io.tr, trbuf);
+    sc_hash_by_pair<NACC>(t, io, trbuf, [&](TrPair& tr) {
         if constexpr (FOLD) {
             const Fe r2 = r * r;
             u32 ew[12];
@@ -357,9 +370,7 @@ __global__ void __launch_bounds__(256) sc_product_base_kernel(ScTables tb, size_
         } else {
             sc_finish_round<SC_PRODUCT, Fp, ChalT>(t, io, round, tr);
         }
-        tr_store(tr, io.tr);
-        *io.counter = 0;
-    }
+    });
 }
 
 // ---- product sumcheck over base-field tables: two challenges folded in one pass -----------------
@@ -445,13 +456,7 @@ __global__ void __launch_bounds__(256) sc_product_base_fold2_kernel(ScTables tb,
     }
     block_sum_words<12>(t, red);
     if (io.xch && threadIdx.x < 32) xch_allreduce_warp<12>(*io.xch, io.xch->seq + round, t);
-    if (threadIdx.x == 0) {
-        Tr tr;
-        tr_load(tr, io.tr, trbuf);
-        sc_finish_round<SC_PRODUCT, Fe, Fe>(t, io, round, tr);
-        tr_store(tr, io.tr);
-        *io.counter = 0;
-    }
+    sc_hash_by_pair<12>(t, io, trbuf, [&](TrPair& tr) { sc_finish_round<SC_PRODUCT, Fe, Fe>(t, io, round, tr); });
 }
 
 // ---- product sumcheck over base-field tables: rounds 0 and 1 in one launch -------------------------------
@@ -500,9 +505,7 @@ __global__ void __launch_bounds__(256) sc_product_base_two_kernel(ScTables tb, s
         for (int k = 0; k < 9; k++) t[k] = add31(t[k], __ldcg(io.partials + (size_t)b * 16 + k));
     }
     block_sum_words<9>(t, red);
-    if (threadIdx.x == 0) {
-        Tr tr;
-        tr_load(tr, io.tr, trbuf);
+    sc_hash_by_pair<9>(t, io, trbuf, [&](TrPair& tr) {
         const u32 l0 = add31(t[0], t[3]), l1 = add31(t[1], t[4]), l2 = add31(t[2], t[5]);
         const u32 m0[3] = {l0, add31(l0, add31(l1, l2)), add31(l0, add31(add31(l1, l1), mul31(4u, l2)))};
         const Fe r = sc_finish_round<SC_PRODUCT, Fp, Fe>(m0, io, round, tr), r2 = r * r;
@@ -514,9 +517,16 @@ __global__ void __launch_bounds__(256) sc_product_base_two_kernel(ScTables tb, s
             to_words(s, m1 + 4 * k);
         }
         sc_finish_round<SC_PRODUCT, Fe, Fe>(m1, io, round + 1, tr);
-        tr_store(tr, io.tr);
-        *io.counter = 0;
-    }
+    });
+}
+
+// Base-field squeezes behind the final evaluations, by warps 0 and 1.
+__device__ __forceinline__ void sc_post_squeezes(TrPair& tr, const ScIO& io, const unsigned char* trbuf) {
+    if (io.post_squeezes == 0) return;
+    if (threadIdx.x < 32) {
+        tr_squeeze_run(tr, io.post_squeezes, [&](u32 q, u32 v) { if (threadIdx.x == 0 && io.post_out) io.post_out[q] = v; });
+        tr_pair_end(tr);
+    } else if (threadIdx.x < 64) tr_pair_help(trbuf);
 }
 
 // ---- single-CTA tail: all remaining rounds and the final evaluations -------------------------
@@ -534,8 +544,9 @@ __global__ void __launch_bounds__(SC_TAIL_THREADS) sc_tail_kernel(ScTables tb, s
 
     ZKB_STAMP_BEGIN
     if (io.dyn_nv) { num_vars = io.dyn_nv[0]; size = size_t(1) << num_vars; }
-    Tr tr;
-    if (threadIdx.x == 0) tr_load(tr, io.tr, trbuf);
+    const int warp = threadIdx.x >> 5;            // warp 0 hashes, warp 1 expands schedules for it (two warps at least)
+    TrPair tr;
+    if (warp == 0) tr_load(tr, io.tr, trbuf);
     ChalT r = zero_of<ChalT>();
     if (pending) from_words(r, io.chal + (size_t)(round - 1) * WC);
     bool in_src = true;           // tables still in their input buffers / input type
@@ -586,10 +597,13 @@ __global__ void __launch_bounds__(SC_TAIL_THREADS) sc_tail_kernel(ScTables tb, s
         }
         block_sum_words<NACC * WC>(w, red);
         if (io.xch && phase == 0 && threadIdx.x < 32) xch_allreduce_warp<NACC * WC>(*io.xch, io.xch->seq + round, w);
-        if (threadIdx.x == 0) {
+        if (warp == 0) {
+#pragma unroll
+            for (int k = 0; k < NACC * WC; k++) w[k] = __shfl_sync(0xffffffffu, w[k], 0);
             ChalT rn = sc_finish_round<KIND, ChalT, ChalT>(w, io, round, tr);
+            tr_pair_end(tr);
             to_words(rn, r_sh);
-        }
+        } else if (warp == 1) tr_pair_help(trbuf);
         __syncthreads();
         from_words(r, r_sh);
         pending = 1;
@@ -633,11 +647,8 @@ __global__ void __launch_bounds__(SC_TAIL_THREADS) sc_tail_kernel(ScTables tb, s
     stop = num_vars;
     }
 
+    sc_post_squeezes(tr, io, trbuf);
     if (threadIdx.x == 0) {
-        for (u32 q = 0; q < io.post_squeezes; q++) {
-            u32 v = tr_squeeze(tr);
-            if (io.post_out) io.post_out[q] = v;
-        }
         tr_store(tr, io.tr);
         // size == 2 here: fold the last challenge in.
 #pragma unroll

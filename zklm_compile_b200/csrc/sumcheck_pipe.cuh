@@ -26,13 +26,23 @@ template <class T> constexpr int PIPE_NW = 9 * Width<T>::W;   // nine coefficien
 
 // Roles.  Warp 0 hashes.  Warps 4, 8, 12 would share warp 0's scheduler (warp w issues on sub-
 // partition w mod 4), its instruction cache and its issue slots; they only join the CTA barriers,
-// so the hash chain has a sub-partition to itself.  The other warps are the workers, numbered
-// 0, 1, 2, ... in warp order.
-__device__ __forceinline__ bool pipe_is_worker(int warp) { return (warp & 3) != 0; }
-__device__ __forceinline__ int pipe_worker_index(int warp) { return warp - 1 - (warp >> 2); }
-__device__ __forceinline__ int pipe_worker_warps() { const int last = (int)(blockDim.x >> 5) - 1; return last - (last >> 2); }
-// Barrier 1 among the worker warps only; blockDim.x is a multiple of 32.
-__device__ __forceinline__ void pipe_worker_barrier() { asm volatile("bar.sync 1, %0;" ::"r"(pipe_worker_warps() * 32) : "memory"); }
+// so the hash chain has a sub-partition to itself.  While a round's tables are long its table pass takes longer than its
+// hash, and all other warps are workers.  From pipe_paired() on warp 1 expands the message schedules instead (TrPair), with the
+// second sub-partition to itself, and the warps of the other two are the workers.  They are numbered 0, 1, 2, ... in warp order.
+struct PipeRole { int index, warps; };           // index below 0: not a worker
+__device__ __forceinline__ PipeRole pipe_role(bool paired) {
+    const int warp = threadIdx.x >> 5, n = blockDim.x >> 5;
+    if (!paired) return PipeRole{(warp & 3) ? warp - 1 - (warp >> 2) : -1, n - 1 - ((n - 1) >> 2)};
+    return PipeRole{(warp & 3) >= 2 ? 2 * (warp >> 2) + (warp & 3) - 2 : -1, 2 * (n >> 2) + ((n & 3) == 3 ? 1 : 0)};
+}
+// n: length of the tables whose message a round hashes.  The line lies where the pass of the workers that are left takes about as
+// long as the shared hash.  Measured on B200, never paired / this line / always: four 4B-shape layers 16.77 / 16.20 / 16.31 ms, the
+// 1024-2048-1024-10 MLP (base field) 1384 / 1352 / 1352 us.
+template <class T> __device__ __forceinline__ bool pipe_paired(size_t n) {
+    return n <= (Width<T>::W == 4 ? 128 : 512) * (size_t)(blockDim.x >> 5);
+}
+// Barrier 1 among the worker warps only.
+__device__ __forceinline__ void pipe_worker_barrier(int warps) { asm volatile("bar.sync 1, %0;" ::"r"(warps * 32) : "memory"); }
 
 // Coefficient sums of the next round over one pair index: quarters (a, b, c, d) of f and g.
 template <class T>
@@ -45,15 +55,15 @@ __device__ __forceinline__ void pipe_accum(T* C, T fa, T fb, T fc, T fd, T ga, T
     C[6] = C[6] + pf * pg;  C[7] = C[7] + pf * qg + pg * qf;  C[8] = C[8] + qf * qg;
 }
 
-// Workers only (see pipe_is_worker; at least two worker warps, so that PIPE_NW threads can add the rows).  Tables of size n at (rf, rg); if `fold`, they are first
+// Workers only.  Tables of size n at (rf, rg); if `fold`, they are first
 // folded with r into size n / 2 at (wf, wg) (in place allowed) and the sums are taken over the
 // folded tables.  Leaves the PIPE_NW summed words in out[] (shared memory) when the result size is >= 4.
 template <class T>
 __device__ __forceinline__ void pipe_worker_pass(const T* rf, const T* rg, T* wf, T* wg, size_t n, bool fold, T r,
-                                                 u32 (*cw)[PIPE_NW<T>], u32* out) {
+                                                 u32 (*cw)[PIPE_NW<T>], u32* out, PipeRole role) {
     constexpr int NW = PIPE_NW<T>;
-    const int worker_warps = pipe_worker_warps();
-    const int wid = pipe_worker_index(threadIdx.x >> 5) * 32 + (threadIdx.x & 31);
+    const int worker_warps = role.warps;
+    const int wid = role.index * 32 + (threadIdx.x & 31);
     const size_t workers = (size_t)worker_warps * 32;
     const size_t m = fold ? n / 2 : n;              // size of the tables the sums run over
     T C[9];
@@ -92,7 +102,7 @@ __device__ __forceinline__ void pipe_worker_pass(const T* rf, const T* rg, T* wf
         u32 w[NW];
 #pragma unroll
         for (int i = 0; i < 9; i++) to_words(C[i], w + Width<T>::W * i);
-        const int lane = threadIdx.x & 31, warp = pipe_worker_index(threadIdx.x >> 5);
+        const int lane = threadIdx.x & 31, warp = role.index;
 #pragma unroll
         for (int k = 0; k < NW; k++) {
 #pragma unroll
@@ -102,11 +112,11 @@ __device__ __forceinline__ void pipe_worker_pass(const T* rf, const T* rg, T* wf
 #pragma unroll
             for (int k = 0; k < NW; k++) cw[warp][k] = w[k];
         }
-        pipe_worker_barrier();
-        if (wid < NW) {
+        pipe_worker_barrier(worker_warps);
+        for (int k = wid; k < NW; k += (int)workers) {
             u32 v = 0;
-            for (int rw = 0; rw < worker_warps; rw++) v = add31(v, cw[rw][wid]);
-            out[wid] = v;
+            for (int rw = 0; rw < worker_warps; rw++) v = add31(v, cw[rw][k]);
+            out[k] = v;
         }
     }
 }
@@ -123,8 +133,9 @@ __global__ void __launch_bounds__(PIPE_THREADS) sc_tail_product_pipe_kernel(ScTa
     __shared__ u32 w_sh[3 * W];
 
     ZKB_STAMP_BEGIN
-    Tr tr;
-    if (threadIdx.x == 0) tr_load(tr, io.tr, trbuf);
+    const int warp = threadIdx.x >> 5;
+    TrPair tr;
+    if (warp == 0) tr_load(tr, io.tr, trbuf);
     T r = zero_of<T>();
     if (pending) from_words(r, io.chal + (size_t)(round - 1) * W);
 
@@ -149,23 +160,35 @@ __global__ void __launch_bounds__(PIPE_THREADS) sc_tail_product_pipe_kernel(ScTa
         block_sum_words<3 * W>(w, red);                 // ends with a CTA barrier: folded tables visible
     }
 
+    if (warp == 0) {
+#pragma unroll
+        for (int i = 0; i < 3 * W; i++) w[i] = __shfl_sync(0xffffffffu, w[i], 0);
+    }
     bool first = true;
     u32 k = round;
     for (;;) {
-        // thread 0 hashes round k; the workers prepare round k + 1 as polynomials in r_k
-        if (threadIdx.x == 0) {
-            T rn = sc_finish_round<SC_PRODUCT, T, T>(w, io, k, tr);
+        // warp 0 hashes round k; the workers prepare round k + 1 as polynomials in r_k
+        const bool paired = pipe_paired<T>(n);
+        const PipeRole role = pipe_role(paired);
+        if (warp == 0) {
+            T rn;
+            if (paired) {
+                rn = sc_finish_round<SC_PRODUCT, T, T>(w, io, k, tr);
+                tr_pair_end(tr);
+            } else rn = sc_finish_round<SC_PRODUCT, T, T>(w, io, k, static_cast<TrWarp&>(tr));
             to_words(rn, r_sh[k & 1]);
-        } else if (pipe_is_worker(threadIdx.x >> 5)) {
-            if (first) pipe_worker_pass(rf, rg, wf, wg, n, false, r, cw, csum[k & 1]);
-            else       pipe_worker_pass(rf, rg, wf, wg, 2 * n, true, r, cw, csum[k & 1]);
+        } else if (paired && warp == 1) {
+            tr_pair_help(trbuf);
+        } else if (role.index >= 0) {
+            if (first) pipe_worker_pass(rf, rg, wf, wg, n, false, r, cw, csum[k & 1], role);
+            else       pipe_worker_pass(rf, rg, wf, wg, 2 * n, true, r, cw, csum[k & 1], role);
         }
         __syncthreads();
         if (!first) { rf = wf; rg = wg; }            // the fold above wrote dst
         first = false;
         from_words(r, r_sh[k & 1]);                  // r_k
         if (n == 2) break;                           // round k was the last one
-        if (threadIdx.x < 32) {                      // three lanes evaluate the three quadratics, lane 0 collects
+        if (warp == 0) {                             // three lanes evaluate the three quadratics, all collect
             if (threadIdx.x < 3) {
                 const u32* c = csum[k & 1] + 3 * W * threadIdx.x;
                 T c0, c1, c2;
@@ -173,21 +196,17 @@ __global__ void __launch_bounds__(PIPE_THREADS) sc_tail_product_pipe_kernel(ScTa
                 to_words(c0 + r * (c1 + r * c2), w_sh + W * threadIdx.x);
             }
             __syncwarp();
-            if (threadIdx.x == 0) {
 #pragma unroll
-                for (int i = 0; i < 3 * W; i++) w[i] = w_sh[i];
-            }
+            for (int i = 0; i < 3 * W; i++) w[i] = w_sh[i];
+            __syncwarp();
         }
         k++;
         n /= 2;
     }
     (void)num_vars;
 
+    sc_post_squeezes(tr, io, trbuf);
     if (threadIdx.x == 0) {
-        for (u32 q = 0; q < io.post_squeezes; q++) {
-            u32 v = tr_squeeze(tr);
-            if (io.post_out) io.post_out[q] = v;
-        }
         tr_store(tr, io.tr);
         // two elements per table remain (folded through r_(k-1)): fold the last challenge in
         T fv = lerp(ld_fe(rf), ld_fe(rf + 1), r), gv = lerp(ld_fe(rg), ld_fe(rg + 1), r);

@@ -195,10 +195,10 @@ __device__ __forceinline__ void sha256_expand_kw(const u32* __restrict__ blk_be,
     }
 }
 
-// Working copy used by the single thread that advances the transcript.  `buf` points to
-// TR_SCRATCH_BYTES of 16-byte-aligned shared memory: the 64-byte message block followed by 64
-// words for the expanded schedule (K + W) of the block being compressed.
-constexpr int TR_SCRATCH_BYTES = 64 + 64 * 4;
+// Working copy used by the thread (Tr) or the warp (TrWarp, TrPair, below) that advances the transcript.  `buf` points to
+// TR_SCRATCH_BYTES of 16-byte-aligned shared memory: the 64-byte message block, then what a pair of warps shares: the 64
+// words K + W of the block being compressed, a digest that is the message, and the order to the second warp.
+constexpr int TR_SCRATCH_BYTES = 64 + 64 * 4 + 64;
 
 struct Tr {
     u32 h[8];
@@ -207,11 +207,146 @@ struct Tr {
     unsigned char* buf;
 };
 
+// ---- a compression shared by two warps ------------------------------------------------------------
+// More than a third of a fused compression's time is the message schedule, which does not depend on the chaining
+// value.  Where a CTA has a warp to spare, that warp (on another scheduler) expands it: the hashing warp writes the
+// message, arrives at a named barrier and runs rounds 0..15, for which it has the words; meanwhile the second warp
+// expands W[16..31] + K and hands them over through a second barrier, then the other 32 through a third.  A schedule
+// word takes it less than a round, so it stays ahead from there on.  The hashing warp runs its code with all lanes in step
+// (they hold the same state), so that the barriers see whole warps.
+// What bounds it is 64 dependent rounds at 27 cycles, and the size of the code: next to the table work of a tail or to
+// other streams' kernels, loops of sixteen rounds for the one warp and of sixteen words for the other are faster than
+// unrolled ones.  Measured on B200, whole calls in us (before, fused in one thread / both warps unrolled / both in loops): four 4B-shape
+// layers 17690 / 19400 / 16200, their verifier 16450 / 16870 / 14920, the 1024-2048-1024-10 MLP 1522 / 1525 / 1352, a sumcheck
+// of 2^12 elements 237 / 225 / 211.
+struct TrWarp : Tr {};           // all lanes of a warp in step, compressing alone
+struct TrPair : TrWarp {};       // with the second warp
+constexpr u32 TRP_KW = 64, TRP_MSG = TRP_KW + 64 * 4, TRP_ORDER = TRP_MSG + 8 * 4;      // byte offsets behind `buf`
+static_assert(TRP_ORDER + 4 <= TR_SCRATCH_BYTES, "scratch of a pair");
+enum : u32 { TRP_STOP = 0, TRP_BLOCK = 1, TRP_DIGEST = 2 };        // orders: leave; expand the block in `buf`; expand a digest || its padding
+constexpr int TRP_BAR_ORDER = 2, TRP_BAR_FIRST = 3, TRP_BAR_REST = 4;    // named barriers (0: the CTA, 1: workers of the pipelined tail)
+template <int B> __device__ __forceinline__ void trp_arrive() { asm volatile("bar.arrive %0, 64;" ::"n"(B) : "memory"); }
+template <int B> __device__ __forceinline__ void trp_sync() { asm volatile("bar.sync %0, 64;" ::"n"(B) : "memory"); }
+__device__ __forceinline__ u32 sh_addr(const void* p) { return (u32)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void sh_ld4(u32 a, u32* o) { asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3]) : "r"(a) : "memory"); }
+__device__ __forceinline__ void sh_st4(u32 a, const u32* v) { asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory"); }
+__device__ __forceinline__ u32 sh_ld(u32 a) { u32 v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory"); return v; }
+__device__ __forceinline__ void sh_st(u32 a, u32 v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+#define ZKB_SHA_RND8_KW(k)                                                                                                                    \
+    ZKB_SHA_RND_KW(a, b, c, d, e, f, g, h, (k)[0]); ZKB_SHA_RND_KW(h, a, b, c, d, e, f, g, (k)[1]); ZKB_SHA_RND_KW(g, h, a, b, c, d, e, f, (k)[2]); \
+    ZKB_SHA_RND_KW(f, g, h, a, b, c, d, e, (k)[3]); ZKB_SHA_RND_KW(e, f, g, h, a, b, c, d, (k)[4]); ZKB_SHA_RND_KW(d, e, f, g, h, a, b, c, (k)[5]); \
+    ZKB_SHA_RND_KW(c, d, e, f, g, h, a, b, (k)[6]); ZKB_SHA_RND_KW(b, c, d, e, f, g, h, a, (k)[7]);
+// The hashing warp's rounds, all lanes; kw[0..15] are its own.
+__device__ __noinline__ Sha8 sha256_rounds_pair(Sha8 hin, const unsigned char* buf) {
+    u32 one = SHA_ONE, minus_one = 0u - SHA_ONE;
+    asm volatile("" : "+r"(one), "+r"(minus_one));
+    const u32 kw = sh_addr(buf) + TRP_KW;
+    u32 a = hin.v[0], b = hin.v[1], c = hin.v[2], d = hin.v[3], e = hin.v[4], f = hin.v[5], g = hin.v[6], h = hin.v[7];
+#pragma unroll 1
+    for (u32 i = 0; i < 4; i++) {
+        if (i == 1) trp_sync<TRP_BAR_FIRST>();
+        if (i == 2) trp_sync<TRP_BAR_REST>();
+        u32 k[16];
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) sh_ld4(kw + 64 * i + 4 * j, k + j);
+        ZKB_SHA_RND8_KW(k)
+        ZKB_SHA_RND8_KW(k + 8)
+    }
+    __syncwarp();
+    Sha8 o;
+    o.v[0] = hin.v[0] + a; o.v[1] = hin.v[1] + b; o.v[2] = hin.v[2] + c; o.v[3] = hin.v[3] + d;
+    o.v[4] = hin.v[4] + e; o.v[5] = hin.v[5] + f; o.v[6] = hin.v[6] + g; o.v[7] = hin.v[7] + h;
+    return o;
+}
+// The block in `buf` (16 little-endian words).
+__device__ __forceinline__ Sha8 sha256_compress_pair(Sha8 hin, const unsigned char* buf) {
+    const u32 sb = sh_addr(buf);
+    sh_st(sb + TRP_ORDER, TRP_BLOCK);
+    __syncwarp();
+    trp_arrive<TRP_BAR_ORDER>();
+    u32 k[16];
+#pragma unroll
+    for (int i = 0; i < 16; i += 4) sh_ld4(sb + 4 * i, k + i);
+#pragma unroll
+    for (int i = 0; i < 16; i++) k[i] = SHA_K[i] + bswap32(k[i]);
+#pragma unroll
+    for (int i = 0; i < 16; i += 4) sh_st4(sb + TRP_KW + 4 * i, k + i);
+    return sha256_rounds_pair(hin, buf);
+}
+// A digest as the whole message, from the initial state.
+__device__ __forceinline__ Sha8 sha256_digest_pair(const Sha8& m, const unsigned char* buf) {
+    const u32 sb = sh_addr(buf);
+    sh_st4(sb + TRP_MSG, m.v); sh_st4(sb + TRP_MSG + 16, m.v + 4);
+    sh_st(sb + TRP_ORDER, TRP_DIGEST);
+    __syncwarp();
+    trp_arrive<TRP_BAR_ORDER>();
+    u32 k[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) k[i] = SHA_K[i] + (i < 8 ? m.v[i & 7] : (i == 8 ? 0x80000000u : (i == 15 ? 256u : 0u)));
+#pragma unroll
+    for (int i = 0; i < 16; i += 4) sh_st4(sb + TRP_KW + 4 * i, k + i);
+    return sha256_rounds_pair(Sha8{{0x6a09e667u, 0xbb67ae85u, 0x3c6ef372u, 0xa54ff53au, 0x510e527fu, 0x9b05688cu, 0x1f83d9abu, 0x5be0cd19u}}, buf);
+}
+// The second warp's part, all lanes: serves compressions until tr_pair_end.  Two words a step: even lanes the even schedule
+// words, odd lanes the odd ones.  With x[j] = W[2j + l] and z[j] = W[2j - 1 + l] (words of the other lane) a step is
+// x[j] = sig1(x[j-1]) + z[j-3] + sig0(z[j-7]) + x[j-8].
+__device__ __forceinline__ u32 sha_sig0(u32 v) { return sha_xor3(rotr32(v, 7), rotr32(v, 18), v >> 3); }
+__device__ __forceinline__ u32 sha_sig1(u32 v) { return sha_xor3(rotr32(v, 17), rotr32(v, 19), v >> 10); }
+__device__ __noinline__ void tr_pair_help(const unsigned char* buf) {
+    const u32 sb = sh_addr(buf), l = threadIdx.x & 1;
+    for (;;) {
+        __syncwarp();
+        trp_sync<TRP_BAR_ORDER>();
+        const u32 order = sh_ld(sb + TRP_ORDER);
+        if (order == TRP_STOP) return;
+        u32 x[8], z[8];
+        z[0] = 0;
+        if (order == TRP_DIGEST) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) x[j] = sh_ld(sb + TRP_MSG + 8 * j + 4 * l);
+#pragma unroll
+            for (int j = 1; j < 4; j++) z[j] = sh_ld(sb + TRP_MSG + 8 * j - 4 + 4 * l);
+            z[4] = sh_ld(sb + TRP_MSG + 28);
+            if (l) z[4] = 0x80000000u;
+            x[4] = l ? 0u : 0x80000000u; x[5] = x[6] = 0; x[7] = l ? 256u : 0u;
+            z[5] = z[6] = z[7] = 0;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; j++) x[j] = bswap32(sh_ld(sb + 8 * j + 4 * l));
+#pragma unroll
+            for (int j = 1; j < 8; j++) z[j] = bswap32(sh_ld(sb + 8 * j - 4 + 4 * l));
+        }
+#pragma unroll 1
+        for (u32 i = 0; i < 3; i++) {
+            u32 kk[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) kk[j] = SHA_K[16 + 16 * i + 2 * j + l];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const u32 v = sha_sig1(x[(j + 7) & 7]) + (z[(j + 5) & 7] + (sha_sig0(z[(j + 1) & 7]) + x[j]));
+                sh_st(sb + TRP_KW + 64 + 64 * i + 8 * j + 4 * l, v + kk[j]);
+                z[j] = __shfl_xor_sync(0xffffffffu, l ? x[(j + 7) & 7] : v, 1);
+                x[j] = v;
+            }
+            if (i == 0) trp_arrive<TRP_BAR_FIRST>();
+        }
+        trp_arrive<TRP_BAR_REST>();
+    }
+}
+// The hashing warp compresses with TrPair only while exactly one other warp of the CTA is in tr_pair_help; this sends it out.  A CTA
+// barrier lies between that and the next such stretch (the second warp still reads the order).
+__device__ __forceinline__ void tr_pair_end(const TrPair& t) {
+    sh_st(sh_addr(t.buf) + TRP_ORDER, TRP_STOP);
+    __syncwarp();
+    trp_arrive<TRP_BAR_ORDER>();
+}
+
 __device__ __forceinline__ void tr_iv(u32 h[8]) {
     h[0] = 0x6a09e667u; h[1] = 0xbb67ae85u; h[2] = 0x3c6ef372u; h[3] = 0xa54ff53au;
     h[4] = 0x510e527fu; h[5] = 0x9b05688cu; h[6] = 0x1f83d9abu; h[7] = 0x5be0cd19u;
 }
-__device__ __forceinline__ void tr_load(Tr& t, const TrState* g, unsigned char* scratch) {
+template <class T>
+__device__ __forceinline__ void tr_load(T& t, const TrState* g, unsigned char* scratch) {
 #pragma unroll
     for (int i = 0; i < 8; i++) t.h[i] = g->h[i];
     t.buflen = g->buflen;
@@ -243,12 +378,28 @@ __device__ __forceinline__ void tr_flush_block(Tr& t) {
     for (int i = 0; i < 8; i++) t.h[i] = h.v[i];
     t.buflen = 0;
 }
-__device__ __forceinline__ void tr_absorb_byte(Tr& t, unsigned char c) {
+__device__ __forceinline__ void tr_flush_block(TrWarp& t) {
+    __syncwarp();
+    tr_flush_block(static_cast<Tr&>(t));
+    __syncwarp();
+}
+__device__ __forceinline__ void tr_flush_block(TrPair& t) {
+    Sha8 h;
+#pragma unroll
+    for (int i = 0; i < 8; i++) h.v[i] = t.h[i];
+    h = sha256_compress_pair(h, t.buf);
+#pragma unroll
+    for (int i = 0; i < 8; i++) t.h[i] = h.v[i];
+    t.buflen = 0;
+}
+template <class T>
+__device__ __forceinline__ void tr_absorb_byte(T& t, unsigned char c) {
     t.buf[t.buflen++] = c;
     t.total++;
     if (t.buflen == 64) tr_flush_block(t);
 }
-__device__ __forceinline__ void tr_absorb_u32(Tr& t, u32 v) {
+template <class T>
+__device__ __forceinline__ void tr_absorb_u32(T& t, u32 v) {
     if ((t.buflen & 3) == 0) {           // aligned fast path: one word store
         *reinterpret_cast<u32*>(t.buf + t.buflen) = v;
         t.buflen += 4;
@@ -263,8 +414,8 @@ __device__ __forceinline__ void tr_absorb_u32(Tr& t, u32 v) {
 }
 // N words at once; when the stream is word-aligned (the common case) this is N plain stores
 // plus at most one compression, instead of N rounds of per-byte bookkeeping.
-template <int N>
-__device__ __forceinline__ void tr_absorb_words(Tr& t, const u32* w) {
+template <int N, class T>
+__device__ __forceinline__ void tr_absorb_words(T& t, const u32* w) {
     static_assert(N <= 16, "at most one block boundary inside");
     if ((t.buflen & 3) == 0) {
         u32* bw = reinterpret_cast<u32*>(t.buf);
@@ -287,20 +438,21 @@ __device__ __forceinline__ void tr_absorb_words(Tr& t, const u32* w) {
         for (int i = 0; i < N; i++) tr_absorb_u32(t, w[i]);
     }
 }
-__device__ __forceinline__ void tr_absorb_fe(Tr& t, Fe v) {
+template <class T>
+__device__ __forceinline__ void tr_absorb_fe(T& t, Fe v) {
     u32 w[4] = {v.x, v.y, v.z, v.w};
     tr_absorb_words<4>(t, w);
 }
-__device__ __forceinline__ void tr_absorb_el(Tr& t, Fp v) { tr_absorb_u32(t, v.v); }
-__device__ __forceinline__ void tr_absorb_el(Tr& t, Fe v) { tr_absorb_fe(t, v); }
-__device__ inline void tr_absorb_bytes(Tr& t, const unsigned char* p, u32 n) {
+template <class T>
+__device__ inline void tr_absorb_bytes(T& t, const unsigned char* p, u32 n) {
     for (u32 i = 0; i < n; i++) tr_absorb_byte(t, p[i]);
 }
 
 // Pad, compress, and restart the stream with the 32-byte digest as its first bytes.  Written
 // without loops whose trip count depends on the position: on a lone thread every dependent
 // instruction costs about 11 cycles, so the zero fill is fourteen predicated stores, not a counted loop.
-__device__ __forceinline__ void tr_finalize_reseed(Tr& t, u32 digest_be[8]) {
+template <class T>
+__device__ __forceinline__ void tr_finalize_reseed(T& t, u32 digest_be[8]) {
     u64 bits = t.total * 8;
     u32 n = t.buflen;
     u32* bw = reinterpret_cast<u32*>(t.buf);
@@ -331,9 +483,20 @@ __device__ __forceinline__ void tr_finalize_reseed(Tr& t, u32 digest_be[8]) {
     t.buflen = 32;
     t.total = 32;
 }
-__device__ __forceinline__ u32 tr_squeeze(Tr& t) {
+// The first of a digest's four little-endian 64-bit windows below 2^64 - 4, reduced mod p; false when there is none.
+__device__ __forceinline__ bool tr_window(const u32* d, u32& v) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        u64 raw = (u64)bswap32(d[2 * c]) | ((u64)bswap32(d[2 * c + 1]) << 32);
+        if (raw < 0xfffffffffffffffcull) { v = red64(raw); return true; }
+    }
+    return false;
+}
+// d: the digest that the stream consists of afterwards.
+template <class T>
+__device__ __forceinline__ u32 tr_squeeze_digest(T& t, u32* d) {
+    u32 v = 0;
     for (int guard = 0; guard < 64; guard++) {        // all four windows rejecting has probability 2^-248
-        u32 d[8];
         if (t.buflen == 32 && t.total == 32) {
             // stream == one 32-byte digest (the state right after a squeeze): the padded block is fixed
             u32* bw = reinterpret_cast<u32*>(t.buf);
@@ -351,21 +514,39 @@ __device__ __forceinline__ u32 tr_squeeze(Tr& t) {
         } else {
             tr_finalize_reseed(t, d);
         }
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            u64 raw = (u64)bswap32(d[2 * c]) | ((u64)bswap32(d[2 * c + 1]) << 32);
-            if (raw < 0xfffffffffffffffcull) return red64(raw);
-        }
+        if (tr_window(d, v)) break;
     }
-    return 0;
+    return v;
 }
-__device__ __forceinline__ Fe tr_squeeze_fe(Tr& t) {
-    Fe r;
-    r.x = tr_squeeze(t); r.y = tr_squeeze(t); r.z = tr_squeeze(t); r.w = tr_squeeze(t);
-    return r;
+template <class T>
+__device__ __forceinline__ u32 tr_squeeze(T& t) { u32 d[8]; return tr_squeeze_digest(t, d); }
+// n squeezes in a row, out(i, value) for each.  Behind the first one each message is the digest before it, which the hashing
+// warp has in registers.
+template <class Out>
+__device__ __forceinline__ void tr_squeeze_run(TrPair& t, u32 n, Out out) {
+    if (n == 0) return;
+    Sha8 d;
+    out(0u, tr_squeeze_digest(t, d.v));
+    if (n == 1) return;
+#pragma unroll 1
+    for (u32 i = 1; i < n; i++) {
+        u32 v = 0;
+        for (int guard = 0; guard < 64; guard++) {
+            d = sha256_digest_pair(d, t.buf);
+            if (tr_window(d.v, v)) break;
+        }
+        out(i, v);
+    }
+    u32* bw = reinterpret_cast<u32*>(t.buf);
+#pragma unroll
+    for (int i = 0; i < 8; i++) bw[i] = bswap32(d.v[i]);
 }
-__device__ __forceinline__ void tr_squeeze_el(Tr& t, Fp& r) { r.v = tr_squeeze(t); }
-__device__ __forceinline__ void tr_squeeze_el(Tr& t, Fe& r) { r = tr_squeeze_fe(t); }
+template <class Out>
+__device__ __forceinline__ void tr_squeeze_run(TrWarp& t, u32 n, Out out) { for (u32 i = 0; i < n; i++) out(i, tr_squeeze(t)); }
+template <class T> __device__ __forceinline__ void tr_squeeze_el(T& t, Fp& r) { r.v = tr_squeeze(t); }
+template <class T> __device__ __forceinline__ void tr_squeeze_el(T& t, Fe& r) {
+    tr_squeeze_run(t, 4, [&](u32 i, u32 v) { if (i == 0) r.x = v; else if (i == 1) r.y = v; else if (i == 2) r.z = v; else r.w = v; });
+}
 
 // Warp-cooperative absorb of `total` u32 words produced by load(g), g in [0, total) (any lane may
 // call load).  `tr` is meaningful in lane 0 only; tile (512 words) and kw (32 * SHA_KW_STRIDE
@@ -426,10 +607,10 @@ __device__ __forceinline__ void tr_absorb_stream_warp(Tr& tr, u32 total, Load lo
 // hash chain: while lane 0 of warp 0 runs the rounds of one batch (up to 32 blocks, about 28 us),
 // warp 1 fetches the next batch's words and expands its schedules into the other half of the
 // double-buffered scratch; the two meet at a CTA barrier per batch.  Called by all 64 threads with
-// identical arguments; `tr` is meaningful in thread 0; `bufw` is the stream buffer (shared
+// identical arguments; `tr` is meaningful in warp 0, the same in all its lanes; `bufw` is the stream buffer (shared
 // memory) that tr.buf points to; tile holds 2 x 512 words, kw 2 x 32 x SHA_KW_STRIDE, bc 1 word.
-template <class Load>
-__device__ __forceinline__ void tr_absorb_stream_2w_aligned(Tr& tr, u32 total, Load load, u32* bufw, u32 have, u32* tile, u32* kw) {
+template <class T, class Load>
+__device__ __forceinline__ void tr_absorb_stream_2w_aligned(T& tr, u32 total, Load load, u32* bufw, u32 have, u32* tile, u32* kw) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     auto produce = [&](u32 slot, u32 have_, u32 pos, u32 nb) {   // warp 1: words [pos, ...) after `have_` buffered ones
         u32* t = tile + slot * 512;
@@ -450,7 +631,7 @@ __device__ __forceinline__ void tr_absorb_stream_2w_aligned(Tr& tr, u32 total, L
         if (next_nb > 32) next_nb = 32;
         if (warp == 1) {
             if (next_nb) produce(slot ^ 1, 0, next_pos, next_nb);
-        } else if (lane == 0) {
+        } else {
             const u32* k = kw + slot * 32 * SHA_KW_STRIDE;
             Sha8 h;
 #pragma unroll
@@ -464,11 +645,11 @@ __device__ __forceinline__ void tr_absorb_stream_2w_aligned(Tr& tr, u32 total, L
     }
     const u32 rest = total - pos;      // fewer than 16 - have words: they stay in the stream buffer
     if (warp == 0) for (u32 j = lane; j < rest; j += 32) bufw[have + j] = load(pos + j);
-    if (threadIdx.x == 0) { tr.buflen = (have + rest) * 4; tr.total += (u64)total * 4; }
+    if (warp == 0) { tr.buflen = (have + rest) * 4; tr.total += (u64)total * 4; }
     __syncthreads();
 }
-template <class Load>
-__device__ __forceinline__ void tr_absorb_stream_2w(Tr& tr, u32 total, Load load, u32* bufw, u32* tile, u32* kw, u32* bc) {
+template <class T, class Load>
+__device__ __forceinline__ void tr_absorb_stream_2w(T& tr, u32 total, Load load, u32* bufw, u32* tile, u32* kw, u32* bc) {
     if (threadIdx.x == 0) bc[0] = tr.buflen;
     __syncthreads();                   // also: thread 0's earlier writes to the stream buffer become visible
     const u32 buflen = bc[0];
@@ -481,7 +662,7 @@ __device__ __forceinline__ void tr_absorb_stream_2w(Tr& tr, u32 total, Load load
     __syncthreads();                   // every thread holds the pending bytes before the buffer is written again
     tr_absorb_stream_2w_aligned(tr, total, [=](u32 g) -> u32 { return __funnelshift_l(g ? load(g - 1) : pend, load(g), sh); },
                                 bufw, have, tile, kw);
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         bufw[tr.buflen >> 2] = load(total - 1) >> (32 - sh);
         tr.buflen += s;
     }

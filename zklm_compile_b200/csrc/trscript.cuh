@@ -37,12 +37,14 @@ __global__ void __launch_bounds__(32) tr_absorb_words_kernel(TrState* st, const 
     tr_absorb_stream_warp(tr, (u32)n, [=](u32 g) -> u32 { return v[g]; }, tile, kw);
     if (threadIdx.x == 0) tr_store(tr, st);
 }
-__global__ void tr_squeeze_kernel(TrState* st, u32* out, u32 count) {
+__global__ void __launch_bounds__(64) tr_squeeze_kernel(TrState* st, u32* out, u32 count) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
-    Tr tr;
+    if (threadIdx.x >= 32) { tr_pair_help(trbuf); return; }
+    TrPair tr;
     tr_load(tr, st, trbuf);
-    for (u32 i = 0; i < count; i++) out[i] = tr_squeeze(tr);
-    tr_store(tr, st);
+    tr_squeeze_run(tr, count, [=](u32 i, u32 v) { if (threadIdx.x == 0) out[i] = v; });
+    tr_pair_end(tr);
+    if (threadIdx.x == 0) tr_store(tr, st);
 }
 
 
@@ -63,6 +65,7 @@ struct TrOp {
     const u32* ptr;   // device source / squeeze destination
     const u32* ptr2;  // TROP_PAIRS_DEV second array
 };
+__device__ __forceinline__ bool tr_op_is_short(u32 kind) { return kind != TROP_WORDS_DEV && kind != TROP_PAIRS_DEV && kind != TROP_BYTES_DEV; }
 constexpr int TRSCRIPT_MAX_OPS = 12;
 constexpr int TRSCRIPT_INLINE = 256;
 struct TrScript {
@@ -78,27 +81,33 @@ __global__ void __launch_bounds__(TRSCRIPT_THREADS) tr_script_kernel(TrState* st
     __shared__ __align__(16) u32 kw[2 * 32 * SHA_KW_STRIDE];
     __shared__ u32 bc[1];
     ZKB_STAMP_BEGIN
-    Tr tr;
+    TrPair tr;
     tr.buf = trbuf; tr.buflen = 0; tr.total = 0;
-    if (threadIdx.x == 0) tr_load(tr, st, trbuf);
-    for (u32 o = 0; o < sc.nops; o++) {
-        const TrOp& op = sc.ops[o];
-        if (op.kind == TROP_BYTES) {
-            if (threadIdx.x == 0) tr_absorb_bytes(tr, sc.inl + op.inline_off, op.n);
-        } else if (op.kind == TROP_SQUEEZE) {
-            if (threadIdx.x == 0) {
-                u32* dst = const_cast<u32*>(op.ptr);
-                for (u32 i = 0; i < op.n; i++) dst[i] = tr_squeeze(tr);
+    if (threadIdx.x < 32) tr_load(tr, st, trbuf);
+    for (u32 o = 0; o < sc.nops;) {
+        u32 stop = o;                      // operations up to the next streamed absorb: the two warps hash them as a pair
+        while (stop < sc.nops && tr_op_is_short(sc.ops[stop].kind)) stop++;
+        if (stop > o) {
+            if (threadIdx.x >= 32) tr_pair_help(trbuf);
+            else {
+                for (; o < stop; o++) {
+                    const TrOp& op = sc.ops[o];
+                    if (op.kind == TROP_BYTES) tr_absorb_bytes(tr, sc.inl + op.inline_off, op.n);
+                    else if (op.kind == TROP_SQUEEZE) {
+                        u32* dst = const_cast<u32*>(op.ptr);
+                        tr_squeeze_run(tr, op.n, [=](u32 i, u32 v) { if (threadIdx.x == 0) dst[i] = v; });
+                    } else if (op.kind == TROP_WORD_DEV_N) tr_absorb_u32(tr, op.ptr[0]);
+                    else {
+                        u32 nb = op.ptr[0];
+                        if (nb > 255) nb = 255;
+                        tr_absorb_bytes(tr, reinterpret_cast<const unsigned char*>(op.ptr + 1), nb);
+                    }
+                }
+                tr_pair_end(tr);
             }
-        } else if (op.kind == TROP_WORD_DEV_N) {
-            if (threadIdx.x == 0) tr_absorb_u32(tr, op.ptr[0]);
-        } else if (op.kind == TROP_BYTES_DEV_N) {
-            if (threadIdx.x == 0) {
-                u32 nb = op.ptr[0];
-                if (nb > 255) nb = 255;
-                tr_absorb_bytes(tr, reinterpret_cast<const unsigned char*>(op.ptr + 1), nb);
-            }
+            o = stop;
         } else {
+            const TrOp& op = sc.ops[o++];
             // streamed absorbs: total logical words
             u32 total = op.kind == TROP_WORDS_DEV ? op.pad : (op.kind == TROP_PAIRS_DEV ? 2 * op.n : op.n / 4);
             const u32 kind = op.kind, n = op.n;

@@ -103,21 +103,24 @@ inline bool bv_parse(const uint8_t* bytes, size_t len, BvParsed& out, size_t* us
 }
 
 // ---- device ------------------------------------------------------------------------------------------
-__global__ void bf_verify_chain_kernel(TrState* st, const u32* __restrict__ words, u32 log_n, const u32* __restrict__ point, u32 n_point,
+__global__ void __launch_bounds__(64) bf_verify_chain_kernel(TrState* st, const u32* __restrict__ words, u32 log_n, const u32* __restrict__ point, u32 n_point,
                                        u32* alpha_out, u32* qidx_out) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
-    if (threadIdx.x) return;
-    Tr tr;
+    if (threadIdx.x >= 32) { tr_pair_help(trbuf); return; }
+    const bool lead = threadIdx.x == 0;
+    TrPair tr;
     tr_load(tr, st, trbuf);
     for (u32 round = 0; round < log_n; round++) {
-        alpha_out[round] = bf_next_alpha(tr, point, n_point, round);
+        const u32 alpha = bf_next_alpha(tr, point, n_point, round);
+        if (lead) alpha_out[round] = alpha;
         const u32* root = words + 4 + 4 * round;
         u32 rw[4] = {root[0], root[1], root[2], root[3]};
         tr_absorb_words<4>(tr, rw);
         const u32 prev_half_mask = (1u << (log_n - round)) - 1;
-        for (u32 q = 0; q < BF_QUERIES; q++) qidx_out[round * BF_QUERIES + q] = tr_squeeze(tr) & prev_half_mask;
+        tr_squeeze_run(tr, BF_QUERIES, [=](u32 q, u32 v) { if (lead) qidx_out[round * BF_QUERIES + q] = v & prev_half_mask; });
     }
-    tr_store(tr, st);
+    tr_pair_end(tr);
+    if (lead) tr_store(tr, st);
 }
 
 template <int KIND>
@@ -269,7 +272,7 @@ inline BvRun basefold_verify_enqueue(zkb_ctx* c, TrState* tr, const BvParsed& pr
     if (kind == NODE_AES_MMO) bf_verify_batch_kernel<NODE_AES_MMO><<<n_trees, 128, 0, fork.side>>>(words, trees, run.result_dev);
     else bf_verify_batch_kernel<NODE_BLAKE3><<<n_trees, 128, 0, fork.side>>>(words, trees, run.result_dev);
     ZKB_LAUNCHED(c);
-    bf_verify_chain_kernel<<<1, 32, exclusive_smem(bf_verify_chain_kernel, c), fork.main>>>(tr, words, log_n, point_dev, n_point, alpha, qidx);
+    bf_verify_chain_kernel<<<1, 64, exclusive_smem(bf_verify_chain_kernel, c), fork.main>>>(tr, words, log_n, point_dev, n_point, alpha, qidx);
     ZKB_LAUNCHED(c);
     const u32 items = log_n * BF_QUERIES;
     bf_verify_fold_kernel<<<(items + 7) / 8, 256, 0, fork.main>>>(words, trees, log_n, alpha, qidx, tb.w_flat, run.result_dev + n_trees);

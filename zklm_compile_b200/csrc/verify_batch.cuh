@@ -152,24 +152,29 @@ inline bool bbv_parse(const uint8_t* bytes, size_t len, BbvParsed& out) {
     return r.ok && r.at == len;
 }
 
-__global__ void bbv_chain_kernel(TrState* st, const u32* __restrict__ words, u32 k, u32 roots_off, u32 batched_off, u32 fold_off, u32 log_n,
+__global__ void __launch_bounds__(64) bbv_chain_kernel(TrState* st, const u32* __restrict__ words, u32 k, u32 roots_off, u32 batched_off, u32 fold_off, u32 log_n,
                                  u32* rho_out, u32* alpha_out, u32* qidx_out) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
-    if (threadIdx.x) return;
-    Tr tr;
+    __shared__ u32 alpha[32];
+    if (threadIdx.x >= 32) { tr_pair_help(trbuf); return; }
+    const bool lead = threadIdx.x == 0;
+    TrPair tr;
     tr_load(tr, st, trbuf);
     for (u32 i = 0; i < 4 * k; i++) tr_absorb_u32(tr, words[roots_off + i]);
-    rho_out[0] = tr_squeeze(tr);
+    const u32 rho = tr_squeeze(tr);
+    if (lead) rho_out[0] = rho;
     for (u32 i = 0; i < 4; i++) tr_absorb_u32(tr, words[batched_off + i]);
-    for (u32 b = 0; b < log_n; b++) alpha_out[b] = tr_squeeze(tr);
+    tr_squeeze_run(tr, log_n, [&](u32 b, u32 v) { alpha[b] = v; if (lead) alpha_out[b] = v; });
+    __syncwarp();
     for (u32 round = 0; round < log_n; round++) {
-        tr_absorb_u32(tr, alpha_out[round]);
+        tr_absorb_u32(tr, alpha[round]);
         for (u32 i = 0; i < 4; i++) tr_absorb_u32(tr, words[fold_off + 4 * round + i]);
         const u32 prev_half_mask = (1u << (log_n - round)) - 1;
-        for (u32 q = 0; q < BF_QUERIES; q++) qidx_out[round * BF_QUERIES + q] = tr_squeeze(tr) & prev_half_mask;
+        tr_squeeze_run(tr, BF_QUERIES, [=](u32 q, u32 v) { if (lead) qidx_out[round * BF_QUERIES + q] = v & prev_half_mask; });
     }
-    for (u32 q = 0; q < BF_QUERIES; q++) tr_squeeze(tr);
-    tr_store(tr, st);
+    tr_squeeze_run(tr, BF_QUERIES, [](u32, u32) {});
+    tr_pair_end(tr);
+    if (lead) tr_store(tr, st);
 }
 
 // Fold consistency of one query with the joined polynomials' contributions (basefold.rs:1014-1082): one warp per (round, query).
@@ -236,7 +241,7 @@ inline BvRun basefold_batch_verify_enqueue(zkb_ctx* c, TrState* tr, const BbvPar
     if (kind == NODE_AES_MMO) bf_verify_batch_kernel<NODE_AES_MMO><<<n_trees, 128, 0, fork.side>>>(words, trees, run.result_dev);
     else bf_verify_batch_kernel<NODE_BLAKE3><<<n_trees, 128, 0, fork.side>>>(words, trees, run.result_dev);
     ZKB_LAUNCHED(c);
-    bbv_chain_kernel<<<1, 32, exclusive_smem(bbv_chain_kernel, c), fork.main>>>(tr, words, pr.k, pr.roots_off, pr.batched_off, pr.fold_off, log_n, rho, alpha, qidx);
+    bbv_chain_kernel<<<1, 64, exclusive_smem(bbv_chain_kernel, c), fork.main>>>(tr, words, pr.k, pr.roots_off, pr.batched_off, pr.fold_off, log_n, rho, alpha, qidx);
     ZKB_LAUNCHED(c);
     const u32 items = log_n * BF_QUERIES;
     bbv_fold_kernel<<<(items + 7) / 8, 256, 0, fork.main>>>(words, trees, log_n, rho, alpha, qidx, tb.w_flat, adds, add_first, add_count, run.result_dev + n_trees);

@@ -187,10 +187,10 @@ struct LvScArgs {
 };
 __device__ __forceinline__ Fe lv_ld(const u32* w) { return Fe{w[0], w[1], w[2], w[3]}; }
 // sumcheck.rs:1477-1553
-__global__ void lv_sumcheck_kernel(TrState* st, const u32* __restrict__ pw, LvScArgs a, u32* ok_out) {
+__global__ void __launch_bounds__(64) lv_sumcheck_kernel(TrState* st, const u32* __restrict__ pw, LvScArgs a, u32* ok_out) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
-    if (threadIdx.x) return;
-    Tr tr;
+    if (threadIdx.x >= 32) { tr_pair_help(trbuf); return; }
+    TrPair tr;                             // all lanes of the warp compute the same
     tr_load(tr, st, trbuf);
     bool ok = true;
     Fe claim = a.claim_slot ? *a.claim_slot : lv_ld(pw + a.claim_off);
@@ -212,11 +212,12 @@ __global__ void lv_sumcheck_kernel(TrState* st, const u32* __restrict__ pw, LvSc
         if (!fe_eq(s0 + s1, claim)) ok = false;
         tr_absorb_fe(tr, s0); tr_absorb_fe(tr, s1); tr_absorb_fe(tr, s2);
         if (a.degree == 3) tr_absorb_fe(tr, s3);
-        const Fe r = tr_squeeze_fe(tr);
+        Fe r;
+        tr_squeeze_el(tr, r);
         if (a.n_chal) {
             if (i >= a.n_chal || !fe_eq(r, lv_ld(pw + a.chal_off + 4 * i))) ok = false;
         }
-        if (a.chal_out) a.chal_out[i] = r;
+        if (a.chal_out && threadIdx.x == 0) a.chal_out[i] = r;
         if (a.degree == 2) {
             // Lagrange basis on 0, 1, 2
             const Fe one = fe_one(), two = Fe{2, 0, 0, 0};
@@ -232,9 +233,12 @@ __global__ void lv_sumcheck_kernel(TrState* st, const u32* __restrict__ pw, LvSc
     Fe prod = lv_ld(pw + a.fin_off);
     for (u32 k = 1; k < a.n_fin; k++) prod = prod * lv_ld(pw + a.fin_off + 4 * k);
     if (!fe_eq(claim, prod)) ok = false;
-    for (u32 q = 0; q < a.post_squeezes; q++) (void)tr_squeeze(tr);
-    tr_store(tr, st);
-    *ok_out = ok ? 1u : 0u;
+    tr_squeeze_run(tr, a.post_squeezes, [](u32, u32) {});
+    tr_pair_end(tr);
+    if (threadIdx.x == 0) {
+        tr_store(tr, st);
+        *ok_out = ok ? 1u : 0u;
+    }
 }
 // compute_eq_at_point_ef(a, b) == expected
 __global__ void lv_eq_check_kernel(const Fe* a, const Fe* b, u32 k, const u32* __restrict__ pw, u32 expect_off, u32* ok_out) {
@@ -301,7 +305,7 @@ inline Fe* lv_sumcheck(LvRun& R, const LvSumcheck& s, u32 degree, u32 claim_off,
     R.require(s.n_rounds <= 40);
     Fe* out = R.slot(s.n_rounds ? s.n_rounds : 1);
     LvScArgs a{s.off, s.n_rounds, degree, claim_off, claim_slot, fin_off, n_fin, s.chal_off, s.n_chal, out, post_squeezes};
-    lv_sumcheck_kernel<<<1, 32, exclusive_smem(lv_sumcheck_kernel, R.c), R.c->stream>>>(R.tr, R.pw, a, R.flag());
+    lv_sumcheck_kernel<<<1, 64, exclusive_smem(lv_sumcheck_kernel, R.c), R.c->stream>>>(R.tr, R.pw, a, R.flag());
     ZKB_LAUNCHED(R.c);
     return out;
 }

@@ -311,7 +311,7 @@ static int32_t squeeze_n(zkb_transcript* t, uint32_t* out, u32 count) {
     ZKB_TRY(c, {
         c->use();
         u32* d = c->status + 8;   // 8 spare words after the status word
-        tr_squeeze_kernel<<<1, 1, 0, c->stream>>>(t->dev, d, count);
+        tr_squeeze_kernel<<<1, 64, 0, c->stream>>>(t->dev, d, count);
         c->launches++;
         ZKB_CUDA(cudaGetLastError());
         ZKB_CUDA(cudaMemcpyAsync(out, d, count * 4, cudaMemcpyDeviceToHost, c->stream));
