@@ -1,0 +1,38 @@
+"""GPU parity of the compressions that two warps share: every split of a tail's warps into hash, helper and workers (the lines at which
+the helper starts lie at 128 or 512 elements a warp), byte-aligned and ragged streams, against the CPU oracle, bit-exact."""
+import numpy as np
+import pytest
+
+import zklm_compile_b200 as zk
+from oracle import pyoracle as O
+
+pytestmark = pytest.mark.gpu
+P = (1 << 31) - 1
+PROVE = {"product": zk.prove_product, "product_ef_full": zk.prove_product_ef_full, "triple": zk.prove_triple, "product_ef": zk.prove_product_ef}
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = zk.Context(0)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("option,kind,threads", [("OPT_PIPE_THREADS", k, t) for k in ("product", "product_ef_full") for t in (96, 128, 160, 224, 256, 512)] +
+                         [("OPT_SINGLE_CTA_THREADS", k, t) for k in ("triple", "product_ef") for t in (64, 96, 1024)])
+def test_tails_match_oracle(ctx, option, kind, threads):
+    rng = np.random.default_rng(threads)
+    ctx.set_option(getattr(ctx, option), threads)
+    try:
+        for nv in (1, 2, 8, 10, 12):
+            label = b"pair"[: nv % 5]                  # the four alignments of the stream
+            tabs = [rng.integers(0, P, (1 << nv, 4) if kind.endswith("full") else 1 << nv, dtype=np.int64).astype(np.uint32)
+                    for _ in range(3 if kind == "triple" else 2)]
+            t, o = zk.Transcript(ctx, label), O.Transcript(label)
+            proof, *finals = PROVE[kind](*tabs, nv, t)
+            ref = O.prove(kind, o, tabs, nv)
+            assert proof.round_polys.reshape(nv, -1).tolist() == ref[0].reshape(nv, -1).tolist()
+            assert proof.challenges.reshape(nv, -1).tolist() == ref[1].reshape(nv, -1).tolist()
+            assert t.squeeze_ef().tolist() == o.squeeze_ef().tolist()
+    finally:
+        ctx.set_option(getattr(ctx, option), 0)

@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(64) bfb_begin_kernel(TrState* st, const uint4*
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     if (threadIdx.x >= 32) { tr_pair_help(trbuf); return; }
     const bool lead = threadIdx.x == 0;
-    TrPair tr;
+    TrChain tr;
     tr_load(tr, st, trbuf);
     uint4 r = *root;
     u32 rw[4] = {r.x, r.y, r.z, r.w};
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(64) bfb_begin_kernel(TrState* st, const uint4*
 __global__ void __launch_bounds__(64) bfb_final_kernel(TrState* st, u32 mask, u32* idx) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     if (threadIdx.x >= 32) { tr_pair_help(trbuf); return; }
-    TrPair tr;
+    TrChain tr;
     tr_load(tr, st, trbuf);
     tr_squeeze_run(tr, BF_QUERIES, [=](u32 q, u32 v) { if (threadIdx.x == 0) idx[q] = v & mask; });
     tr_pair_end(tr);

@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(64) bf_chain_kernel(const __grid_constant__ Bf
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     if (threadIdx.x >= 32) { tr_pair_help(trbuf); return; }
     const bool lead = threadIdx.x == 0;
-    TrPair tr;
+    TrChain tr;
     tr_load(tr, a.tr, trbuf);
     for (u32 round = a.first; round < a.first + a.count; round++) {
         const BfRound& p = a.r[round];

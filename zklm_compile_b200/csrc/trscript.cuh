@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(32) tr_absorb_words_kernel(TrState* st, const 
 __global__ void __launch_bounds__(64) tr_squeeze_kernel(TrState* st, u32* out, u32 count) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     if (threadIdx.x >= 32) { tr_pair_help(trbuf); return; }
-    TrPair tr;
+    TrChain tr;
     tr_load(tr, st, trbuf);
     tr_squeeze_run(tr, count, [=](u32 i, u32 v) { if (threadIdx.x == 0) out[i] = v; });
     tr_pair_end(tr);

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(64) bf_verify_chain_kernel(TrState* st, const 
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     if (threadIdx.x >= 32) { tr_pair_help(trbuf); return; }
     const bool lead = threadIdx.x == 0;
-    TrPair tr;
+    TrChain tr;
     tr_load(tr, st, trbuf);
     for (u32 round = 0; round < log_n; round++) {
         const u32 alpha = bf_next_alpha(tr, point, n_point, round);

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(64) bbv_chain_kernel(TrState* st, const u32* _
     __shared__ u32 alpha[32];
     if (threadIdx.x >= 32) { tr_pair_help(trbuf); return; }
     const bool lead = threadIdx.x == 0;
-    TrPair tr;
+    TrChain tr;
     tr_load(tr, st, trbuf);
     for (u32 i = 0; i < 4 * k; i++) tr_absorb_u32(tr, words[roots_off + i]);
     const u32 rho = tr_squeeze(tr);

@@ -190,7 +190,7 @@ __device__ __forceinline__ Fe lv_ld(const u32* w) { return Fe{w[0], w[1], w[2], 
 __global__ void __launch_bounds__(64) lv_sumcheck_kernel(TrState* st, const u32* __restrict__ pw, LvScArgs a, u32* ok_out) {
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     if (threadIdx.x >= 32) { tr_pair_help(trbuf); return; }
-    TrPair tr;                             // all lanes of the warp compute the same
+    TrChain tr;                             // all lanes of the warp compute the same
     tr_load(tr, st, trbuf);
     bool ok = true;
     Fe claim = a.claim_slot ? *a.claim_slot : lv_ld(pw + a.claim_off);
