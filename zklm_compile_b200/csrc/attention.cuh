@@ -16,6 +16,7 @@
 // contiguous buffer whose word order is the stream the caller's transcript absorbs after the rows.
 #pragma once
 #include "engine.cuh"
+#include "host_sha.cuh"
 #include "logup.cuh"
 
 namespace zkb {
@@ -448,14 +449,23 @@ inline u32 att_heads_per_group(size_t num_heads, size_t num_kv_heads) {
     if (num_heads % num_kv_heads) throw ArgFail{ZKB_E_ARG, "attention: num_q_heads must be divisible by num_kv_heads"};
     return (u32)(num_heads / num_kv_heads);
 }
+// What the caller's transcript absorbs in front of the rows.
+struct AttHead {
+    u32 w[4], n = 0;
+    AttHead(u32 num_heads, u32 num_kv_heads, u32 S, u32 D) {
+        w[n++] = num_heads;
+        if (num_kv_heads) w[n++] = num_kv_heads;
+        w[n++] = S; w[n++] = D;
+    }
+};
 inline void attention_forward_enqueue(zkb_ctx* c, const u32* q, const u32* k, const u32* v, u32 num_heads, u32 num_kv_heads, u32 S, u32 D,
                                       const u32* table_out, u32 n_table, u32* attn_out) {
     AttArgs A{q, k, v, table_out, n_table, attn_out, nullptr, nullptr, c->status, 0, att_heads_per_group(num_heads, num_kv_heads), num_kv_heads != 0};
     att_launch(c, c->stream, A, att_layout(S, D), num_heads * S);
 }
-// The whole proof: the forward pass writes the scores | outputs stream, after which the row proofs (every SM but
-// one, for milliseconds) and the caller's transcript absorbing that stream (one thread, one SM, one SHA-256 block
-// after the other) do not depend on each other, so the rows run on the context's second stream.
+// The whole proof: the forward pass writes the scores | outputs stream, after which the row proofs (milliseconds of every SM) and the
+// caller's transcript absorbing that stream (one SHA-256 block after the other) do not depend on each other, so the rows run on the
+// context's second stream.  A long stream, which the proof brings to the host anyway, is absorbed there meanwhile (HostAbsorb).
 // host_rec / host_bind: page-locked destinations of the records and of the scores | outputs stream.
 inline AttRun attention_prove_enqueue(zkb_ctx* c, TrState* tr, const u32* q, const u32* k, const u32* v, u32 num_heads, u32 num_kv_heads, u32 S, u32 D,
                                       const u32* table_out, u32 n_table, u32* attn_out, u32* host_rec, u32* host_bind) {
@@ -477,17 +487,22 @@ inline AttRun attention_prove_enqueue(zkb_ctx* c, TrState* tr, const u32* q, con
         return R;
     }
     AttArgs F{q, k, v, table_out, n_table, attn_out, R.bind, nullptr, c->status, 0, hpg, gqa};
+    const HostAbsorb host(c, tr, (size_t)R.rows * (S + D));
+    host.begin();
     att_launch(c, c->stream, F, R.L, R.rows);
     ZKB_CUDA(cudaMemcpyAsync(host_bind, R.bind, (size_t)R.rows * (S + D) * 4, cudaMemcpyDeviceToHost, c->stream));
     SideFork fork(c, !in_order, 0);
     AttArgs A{q, k, v, table_out, n_table, nullptr, nullptr, R.rec, c->status, 1, hpg, gqa};
     att_launch(c, fork.side, A, R.L, R.rows);
     ZKB_CUDA(cudaMemcpyAsync(host_rec, R.rec, (size_t)R.rows * R.L.words * 4, cudaMemcpyDeviceToHost, fork.side));
-    {   // the dimensions, then every row's scores and outputs (attention.rs:140-143, 254-265)
+    // the dimensions, then every row's scores and outputs (attention.rs:140-143, 254-265; the second one for GQA: 403-406)
+    const AttHead head(num_heads, num_kv_heads, S, D);
+    if (host.on) {
+        ZKB_CUDA(cudaStreamSynchronize(c->stream));
+        host.finish(head.w, head.n, host_bind, (size_t)R.rows * (S + D));
+    } else {
         ScriptBuilder sb;
-        sb.word(num_heads);
-        if (gqa) sb.word(num_kv_heads);                         // attention.rs:403-406
-        sb.word(S); sb.word(D);
+        for (u32 i = 0; i < head.n; i++) sb.word(head.w[i]);
         sb.words_dev(R.bind, (u32)((size_t)R.rows * (S + D)));
         sb.run(c, tr);
     }

@@ -160,6 +160,12 @@ struct zkb_ctx {
         }
         return stage;
     }
+    // Page-locked copy of a transcript that is advanced on the host (HostAbsorb).
+    zkb::TrState* tr_host = nullptr;
+    zkb::TrState* transcript_host() {
+        if (!tr_host) ZKB_CUDA(cudaHostAlloc(&tr_host, sizeof(zkb::TrState), cudaHostAllocDefault));
+        return tr_host;
+    }
     cudaStream_t side = nullptr;
     std::vector<cudaEvent_t> side_ev;
     cudaStream_t side_stream() {

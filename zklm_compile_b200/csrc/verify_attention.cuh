@@ -360,16 +360,20 @@ inline AvRun attention_verify_enqueue(zkb_ctx* c, TrState* tr, const AvParsed& p
     u64 n64 = L.S;
     memcpy(pre + 23, &n64, 8);
     const bool in_order = c->opt_bf_in_order || c->capturing || !tr;       // without a transcript to advance there is nothing to overlap
+    const HostAbsorb host(c, tr, pr.bind.size());
+    host.begin();
     SideFork fork(c, !in_order, 0);
     AvArgs A{k, v, rec, bind, run.result_dev, att_heads_per_group(pr.num_heads, num_kv_heads), num_kv_heads != 0};
     const int threads = c->opt_att_threads ? c->opt_att_threads : ((L.s_pad >= 512 || L.d_pad > 128) ? 256 : 128);
     attention_verify_kernel<<<run.rows, threads, smem, fork.side>>>(A, L, b3_prefix(pre, 31));
     ZKB_LAUNCHED(c);
-    if (tr) {
+    const AttHead head(pr.num_heads, num_kv_heads, pr.S, pr.D);
+    if (host.on) {
+        ZKB_CUDA(cudaStreamSynchronize(c->stream));
+        host.finish(head.w, head.n, pr.bind.data(), pr.bind.size());
+    } else if (tr) {
         ScriptBuilder sb;
-        sb.word(pr.num_heads);
-        if (num_kv_heads) sb.word(num_kv_heads);
-        sb.word(pr.S); sb.word(pr.D);
+        for (u32 i = 0; i < head.n; i++) sb.word(head.w[i]);
         sb.words_dev(bind, (u32)pr.bind.size());
         sb.run(c, tr);
     }

@@ -89,6 +89,7 @@ void zkb_ctx_destroy(zkb_ctx* c) {
     for (cudaEvent_t e : c->side_ev) cudaEventDestroy(e);
     if (c->side) cudaStreamDestroy(c->side);
     if (c->stage) cudaFreeHost(c->stage);
+    if (c->tr_host) cudaFreeHost(c->tr_host);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
 }
