@@ -36,3 +36,21 @@ def test_tails_match_oracle(ctx, option, kind, threads):
             assert t.squeeze_ef().tolist() == o.squeeze_ef().tolist()
     finally:
         ctx.set_option(getattr(ctx, option), 0)
+
+
+@pytest.mark.parametrize("heads,seq,d", [(1, 31, 2), (2, 16, 16), (3, 21, 17)])
+def test_attention_transcript_at_the_host_absorb_line(ctx, heads, seq, d):
+    """Streams of 1023, 1024 and 2394 words: the caller's transcript absorbs them on the device below 1024 words, on the host from there on."""
+    from zklm_compile_b200 import attention, tables
+    rng = np.random.default_rng(seq)
+    q, k = (np.mod(rng.integers(-1, 2, heads * seq * d), P).astype(np.uint32) for _ in range(2))
+    v = rng.integers(0, P, heads * seq * d, dtype=np.int64).astype(np.uint32)
+    table = tables.build_exp_table(100)
+    for label in (b"", b"abc"):                        # an aligned stream and a ragged one
+        t, o = zk.Transcript(ctx, label), O.Transcript(label)
+        proof = attention.prove_row_attention(q, k, v, heads, seq, d, table, t)
+        ref, status = O.prove_row_attention(o, q, k, v, heads, seq, d, table)
+        assert status == 0 and bytes(proof) == bytes(ref)
+        t2 = zk.Transcript(ctx, label)
+        assert attention.verify_row_attention(proof, k, v, heads, seq, d, t2)
+        assert t.squeeze_ef().tolist() == o.squeeze_ef().tolist() == t2.squeeze_ef().tolist()

@@ -78,7 +78,7 @@ inline bool cpu_has_sha() {
 inline void sha256_blocks_host(u32* st, const unsigned char* p, size_t blocks) {
 #if defined(__x86_64__)
     static const bool ni = cpu_has_sha();
-    if (ni) return sha256_blocks_ni(st, p, blocks);
+    if (ni) { sha256_blocks_ni(st, p, blocks); return; }
 #endif
     sha256_blocks_plain(st, p, blocks);
 }
