@@ -436,10 +436,28 @@ inline u32 bf_chain_rounds(u32 round, u32 log_n) {
     return n < log_n - round ? n : log_n - round;
 }
 
+// One half of a polynomial's codeword and its tree; nothing in it depends on the transcript.
+struct BfCommit { u32* cw = nullptr; uint4* tree = nullptr; };
+inline size_t bf_commit_bytes(u32 log_n) { return (size_t(4) << log_n) + 256 + mk_node_count(log_n) * 16 + 16; }
+inline BfCommit bf_commit_place(void* mem, u32 log_n) {
+    const size_t cw = ((size_t(4) << log_n) + 255) & ~size_t(255);
+    return BfCommit{(u32*)mem, (uint4*)((char*)mem + cw)};
+}
+inline void bf_commit_enqueue(zkb_ctx* c, CoefSrc src, u32 log_n, int kind, const BfTables& tb, BfCommit to) {
+    c->prof_mark();
+    bf_encode(c, src, log_n, tb, to.cw, false);
+    c->prof_mark();
+    MkFold none{};
+    none.doubled = 1;
+    mk_build(c, kind, MK_VALUES, to.cw, size_t(1) << log_n, log_n, to.tree, none);
+    c->prof_mark();
+}
+
 // Enqueue commit + opening of the polynomial `src` (num_coeffs live coefficients, padded view of
-// 2^log_n) at the device-resident point.  The transcript first absorbs the commitment root.
+// 2^log_n) at the device-resident point.  The transcript first absorbs the commitment root.  `made`: the commitment, if it
+// has been made already.
 inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t num_coeffs, u32 log_n, const u32* point_dev, u32 n_point,
-                                  int kind) {
+                                  int kind, const BfCommit* made = nullptr) {
     if (log_n < 1 || log_n > 28) throw ArgFail{ZKB_E_TOO_LARGE, "basefold: log_n out of range"};
     if (kind != NODE_BLAKE3 && kind != NODE_AES_MMO) throw ArgFail{ZKB_E_ARG, "unknown node hash"};
     if (kind == NODE_AES_MMO) aes_tables_upload();
@@ -451,11 +469,12 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
     // absorbed, not squeezed: basefold.rs:508-513), so the folds and trees of those rounds do not wait for
     // the transcript: they run ahead on a second stream, each round into buffers of its own, while the
     // context's stream runs the hash chain (root absorb, 24 query squeezes) and the path gathers behind them.
-    const bool ahead = n_point >= log_n && !c->opt_bf_in_order && !c->capturing;
-    u32* cwA = (u32*)c->scratch(n_pad * 4);
+    const bool ahead = n_point >= log_n && !c->opt_bf_in_order;
+    const BfCommit commit = made ? *made : bf_commit_place(c->scratch(bf_commit_bytes(log_n)), log_n);
+    u32* cwA = commit.cw;
     u32* cwB = ahead ? nullptr : (u32*)c->scratch(n_pad / 2 * 4);
     u32* eval = (u32*)c->scratch((n_pad / 2 + 4) * 4);
-    uint4* treeA = (uint4*)c->scratch(mk_node_count(log_n) * 16 + 16);
+    uint4* treeA = commit.tree;
     uint4* treeB = ahead ? nullptr : (uint4*)c->scratch(mk_node_count(log_n) * 16 + 16);
     u32* alpha = (u32*)c->scratch((log_n + 1) * 4);
     std::vector<u32*> cws{cwA};            // the folded codeword of each round: the first fold's is the codeword's half itself
@@ -467,13 +486,7 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
         }
     }
 
-    c->prof_mark();
-    bf_encode(c, src, log_n, tb, cwA, false);
-    c->prof_mark();
-    MkFold none{};
-    none.doubled = 1;
-    mk_build(c, kind, MK_VALUES, cwA, n_pad, log_n, treeA, none);
-    c->prof_mark();
+    if (!made) bf_commit_enqueue(c, src, log_n, kind, tb, commit);
     SideFork fork(c, ahead, log_n);
     pd.root_off = c->rec_alloc(4);
     bf_begin_kernel<<<1, 1, 0, c->stream>>>(tr, treeA + mk_node_count(log_n), point_dev, n_point, alpha, c->rec_dev + pd.root_off);

@@ -172,6 +172,17 @@ struct zkb_ctx {
         if (!side) ZKB_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
         return side;
     }
+    // A stream one priority above the second stream's, for a hash chain that runs beside wide kernels: at equal priority all blocks of
+    // the wide kernel that came first are placed before the chain's next one-block launch.
+    cudaStream_t lifted = nullptr;
+    cudaStream_t lifted_stream() {
+        if (!lifted) {
+            int lo = 0, hi = 0;
+            ZKB_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+            ZKB_CUDA(cudaStreamCreateWithPriority(&lifted, cudaStreamNonBlocking, hi < lo ? lo - 1 : lo));
+        }
+        return lifted;
+    }
     cudaEvent_t side_event(size_t i) {
         while (side_ev.size() <= i) {
             cudaEvent_t e;

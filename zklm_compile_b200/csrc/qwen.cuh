@@ -229,16 +229,25 @@ inline void qwen_prove_launches(zkb_qwen_layer* L, zkb_qwen_layer::Pending& P) {
         sb.words_dev(L->roots_dev, 64);
         sb.run(c, tr);
     }
+    // the eight matrices in the order of their proofs
+    BfAhead commits(c, L->node_hash);
+    if (L->bind_mode == BIND_PCS_FULL) {
+        const struct { int w; u32 m, n; } order[8] = {{W_Q, d.q_dim(), dm}, {W_K, d.k_dim(), dm}, {W_V, d.v_dim(), dm}, {W_O, dm, aod},
+                                                      {W_GPROJ, aod, dm}, {W_GATE, d.d_ff, dm}, {W_UP, d.d_ff, dm}, {W_DOWN, dm, d.d_ff}};
+        for (auto& o : order) commits.add(L->w[o.w], o.m, o.n);
+        commits.start();
+    }
+    BfAhead* ahead = L->bind_mode == BIND_PCS_FULL ? &commits : nullptr;
     P.norm1 = prove_rmsnorm_ef(c, tr, L->norm1_x, L->w[W_NORM1], L->norm1_out, dm, L->n1_scalars);
-    P.mq = prove_matmul_succinct_ef(c, tr, L->w[W_Q], L->norm1_out, L->q, d.q_dim(), dm, L->bind_mode, L->node_hash);
-    P.mk = prove_matmul_succinct_ef(c, tr, L->w[W_K], L->norm1_out, L->k, d.k_dim(), dm, L->bind_mode, L->node_hash);
-    P.mv = prove_matmul_succinct_ef(c, tr, L->w[W_V], L->norm1_out, L->v, d.v_dim(), dm, L->bind_mode, L->node_hash);
+    P.mq = prove_matmul_succinct_ef(c, tr, L->w[W_Q], L->norm1_out, L->q, d.q_dim(), dm, L->bind_mode, L->node_hash, ahead);
+    P.mk = prove_matmul_succinct_ef(c, tr, L->w[W_K], L->norm1_out, L->k, d.k_dim(), dm, L->bind_mode, L->node_hash, ahead);
+    P.mv = prove_matmul_succinct_ef(c, tr, L->w[W_V], L->norm1_out, L->v, d.v_dim(), dm, L->bind_mode, L->node_hash, ahead);
     P.seq1 = c->rec_alloc(2);
     seq1_consistency_kernel<<<1, c->single_cta_threads(), 0, c->stream>>>(tr, L->attn_out, aod, log2_ceil_u(aod), L->v, d.v_dim(), log2_ceil_u(d.v_dim()),
                                                       d.is_gqa() ? 1u : 0u, log2_ceil_u(d.nkv), log2_ceil_u(d.d_head), c->rec_dev + P.seq1);
     ZKB_LAUNCHED(c);
-    P.mo = prove_matmul_succinct_ef(c, tr, L->w[W_O], L->gated_attn, L->gated_out, dm, aod, L->bind_mode, L->node_hash);
-    P.mg = prove_matmul_succinct_ef(c, tr, L->w[W_GPROJ], L->norm1_out, L->g_raw, aod, dm, L->bind_mode, L->node_hash);
+    P.mo = prove_matmul_succinct_ef(c, tr, L->w[W_O], L->gated_attn, L->gated_out, dm, aod, L->bind_mode, L->node_hash, ahead);
+    P.mg = prove_matmul_succinct_ef(c, tr, L->w[W_GPROJ], L->norm1_out, L->g_raw, aod, dm, L->bind_mode, L->node_hash, ahead);
     // prove_sigmoid_gate_ef(gate = g_q, gate_sigmoid = g_sig, input = attn_out, output = gated_attn)
     P.sig_gate = prove_gate_ef(c, tr, L->sigmoid, L->n_table, L->g_q, L->g_sig, L->attn_out, L->g_sig, L->gated_attn, aod);
     const u32 log_d = log2_ceil_u(dm);
@@ -246,14 +255,15 @@ inline void qwen_prove_launches(zkb_qwen_layer* L, zkb_qwen_layer::Pending& P) {
     { ScriptBuilder sb; sb.squeeze(c->rec_dev + P.res1_point, 4 * log_d); sb.run(c, tr); }
     P.res1 = prove_add_ef(c, tr, L->x, L->gated_out, L->h, dm, (const Fe*)(c->rec_dev + P.res1_point), log_d);
     P.norm2 = prove_rmsnorm_ef(c, tr, L->norm2_x, L->w[W_NORM2], L->norm2_out, dm, L->n2_scalars);
-    P.mgate = prove_matmul_succinct_ef(c, tr, L->w[W_GATE], L->norm2_out, L->gate_raw, d.d_ff, dm, L->bind_mode, L->node_hash);
-    P.mup = prove_matmul_succinct_ef(c, tr, L->w[W_UP], L->norm2_out, L->up, d.d_ff, dm, L->bind_mode, L->node_hash);
+    P.mgate = prove_matmul_succinct_ef(c, tr, L->w[W_GATE], L->norm2_out, L->gate_raw, d.d_ff, dm, L->bind_mode, L->node_hash, ahead);
+    P.mup = prove_matmul_succinct_ef(c, tr, L->w[W_UP], L->norm2_out, L->up, d.d_ff, dm, L->bind_mode, L->node_hash, ahead);
     // prove_swiglu_ef(gate = gate_q, gate_silu, up, output = swiglu): hadamard(gate_silu, up)
     P.swiglu = prove_gate_ef(c, tr, L->silu, L->n_table, L->gate_q, L->gate_silu, L->gate_silu, L->up, L->swiglu, d.d_ff);
-    P.mdown = prove_matmul_succinct_ef(c, tr, L->w[W_DOWN], L->swiglu, L->down, dm, d.d_ff, L->bind_mode, L->node_hash);
+    P.mdown = prove_matmul_succinct_ef(c, tr, L->w[W_DOWN], L->swiglu, L->down, dm, d.d_ff, L->bind_mode, L->node_hash, ahead);
     P.res2_point = c->rec_alloc(4 * (size_t)log_d);
     { ScriptBuilder sb; sb.squeeze(c->rec_dev + P.res2_point, 4 * log_d); sb.run(c, tr); }
     P.res2 = prove_add_ef(c, tr, L->h, L->down, L->out, dm, (const Fe*)(c->rec_dev + P.res2_point), log_d);
+    commits.done();
     ZKB_CUDA(cudaGetLastError());
 }
 

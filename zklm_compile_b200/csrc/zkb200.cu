@@ -90,6 +90,7 @@ void zkb_ctx_destroy(zkb_ctx* c) {
     if (c->side) cudaStreamDestroy(c->side);
     if (c->stage) cudaFreeHost(c->stage);
     if (c->tr_host) cudaFreeHost(c->tr_host);
+    if (c->lifted) cudaStreamDestroy(c->lifted);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
 }
