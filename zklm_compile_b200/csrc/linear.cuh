@@ -36,6 +36,7 @@ __device__ __forceinline__ Fe eq_at_index<Fe>(const Fe* r, u32 k, size_t idx) {
 }
 template <class T>
 __global__ void eq_evals_kernel(const T* __restrict__ r, u32 k, T* out) {
+    pdl_small_prologue();
     size_t n = size_t(1) << k;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         st_fe(out + i, eq_at_index<T>(r, k, i));

@@ -225,7 +225,7 @@ inline LayerNormRec prove_layernorm_sqr(zkb_ctx* c, TrState* tr, const u32* xc, 
     u32* gc_point = (u32*)c->scratch((size_t)k * 4 + 16);
     { ScriptBuilder sb; sb.squeeze(gc_point, k); sb.run(c, tr); }
     Fp* eq = (Fp*)c->scratch(n * 4 + 16);
-    eq_evals_kernel<Fp><<<grid_for(c, n), 256, 0, c->stream>>>((const Fp*)gc_point, k, eq);
+    chain_launch(c, eq_evals_kernel<Fp>, grid_for(c, n), 256, 0, (const Fp*)gc_point, k, eq);
     ZKB_LAUNCHED(c);
     const u32* tgp[3] = {(const u32*)eq, g, nullptr};
     R.g_prod = sumcheck_enqueue(c, tr, ZKB_SC_PRODUCT, tgp, k);
@@ -238,7 +238,7 @@ inline LayerNormRec prove_layernorm_sqr(zkb_ctx* c, TrState* tr, const u32* xc, 
     u32* sq_point = (u32*)c->scratch((size_t)k * 4 + 16);
     { ScriptBuilder sb; sb.squeeze(sq_point, k); sb.run(c, tr); }
     Fp* eq2 = (Fp*)c->scratch(n * 4 + 16);
-    eq_evals_kernel<Fp><<<grid_for(c, n), 256, 0, c->stream>>>((const Fp*)sq_point, k, eq2);
+    chain_launch(c, eq_evals_kernel<Fp>, grid_for(c, n), 256, 0, (const Fp*)sq_point, k, eq2);
     ZKB_LAUNCHED(c);
     const u32* ths[3] = {(const u32*)eq2, h, h};
     R.h_sq = sumcheck_enqueue(c, tr, ZKB_SC_TRIPLE, ths, k);
@@ -303,14 +303,14 @@ inline ReluRec prove_relu(zkb_ctx* c, TrState* tr, const u32* z, u32 n_valid, co
     }
     R.a_eval = prove_mle_eval_base(c, tr, a, r_point, k, "relu-eval", root_dev);
     Fp* eq = (Fp*)c->scratch(n * 4 + 16);
-    eq_evals_kernel<Fp><<<grid_for(c, n), 256, 0, c->stream>>>((const Fp*)r_point, k, eq);
+    chain_launch(c, eq_evals_kernel<Fp>, grid_for(c, n), 256, 0, (const Fp*)r_point, k, eq);
     ZKB_LAUNCHED(c);
     const u32* t1[3] = {(const u32*)eq, b, zp};
     R.product = sumcheck_enqueue(c, tr, ZKB_SC_TRIPLE, t1, k);
     u32* r2 = (u32*)c->scratch((size_t)k * 4 + 16);
     { ScriptBuilder sb; sb.squeeze(r2, k); sb.run(c, tr); }
     Fp* eq2 = (Fp*)c->scratch(n * 4 + 16);
-    eq_evals_kernel<Fp><<<grid_for(c, n), 256, 0, c->stream>>>((const Fp*)r2, k, eq2);
+    chain_launch(c, eq_evals_kernel<Fp>, grid_for(c, n), 256, 0, (const Fp*)r2, k, eq2);
     ZKB_LAUNCHED(c);
     const u32* t2[3] = {(const u32*)eq2, b, omb};
     R.boolean = sumcheck_enqueue(c, tr, ZKB_SC_TRIPLE, t2, k);

@@ -20,6 +20,7 @@ struct WidenEqArgs {
     u32 k;
 };
 __global__ void widen_eq_kernel(WidenEqArgs a) {
+    pdl_small_prologue();
     const size_t n = size_t(1) << a.k;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         for (u32 t = 0; t < a.nsrc; t++) {

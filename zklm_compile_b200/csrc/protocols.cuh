@@ -70,7 +70,7 @@ inline EvalRec prove_mle_eval_ef_base(zkb_ctx* c, TrState* tr, const u32* w, u32
     Fe* wef = (Fe*)c->scratch(n * 16);
     WidenEqArgs a{};
     a.src[0] = w; a.dst[0] = wef; a.len[0] = len; a.nsrc = 1; a.point = point; a.eq_out = eq; a.k = k;
-    widen_eq_kernel<<<grid_for(c, n), 256, 0, c->stream>>>(a);
+    chain_launch(c, widen_eq_kernel, grid_for(c, n), 256, 0, a);
     ZKB_LAUNCHED(c);
     const u32* tabs[3] = {(const u32*)eq, (const u32*)wef, nullptr};
     ScOpts o;
@@ -84,7 +84,7 @@ inline EvalRec prove_mle_eval_ef_base(zkb_ctx* c, TrState* tr, const u32* w, u32
 inline EvalRec prove_mle_eval_ef_ef(zkb_ctx* c, TrState* tr, Fe* w_ef, const Fe* point, u32 k) {
     size_t n = size_t(1) << k;
     Fe* eq = (Fe*)c->scratch(n * 16);
-    eq_evals_kernel<Fe><<<grid_for(c, n), 256, 0, c->stream>>>(point, k, eq);
+    chain_launch(c, eq_evals_kernel<Fe>, grid_for(c, n), 256, 0, point, k, eq);
     ZKB_LAUNCHED(c);
     const u32* tabs[3] = {(const u32*)eq, (const u32*)w_ef, nullptr};
     ScOpts o;
@@ -227,7 +227,7 @@ inline MatmulRec prove_matmul_succinct_ef(zkb_ctx* c, TrState* tr, const u32* W,
     }
     // eq table over the rows, then the one pass over W                     (matmul.rs:743-835)
     Fe* eq_r = (Fe*)c->scratch(m_pad * 16);
-    eq_evals_kernel<Fe><<<grid_for(c, m_pad), 256, 0, c->stream>>>((const Fe*)r_dev, R.log_m, eq_r);
+    chain_launch(c, eq_evals_kernel<Fe>, grid_for(c, m_pad), 256, 0, (const Fe*)r_dev, R.log_m, eq_r);
     ZKB_LAUNCHED(c);
     Fe* w_partial = (Fe*)c->scratch(n_pad * 16);
     {
@@ -312,7 +312,7 @@ inline EvalRec prove_mle_eval_base(zkb_ctx* c, TrState* tr, const u32* w, const 
     }
     size_t n = size_t(1) << k;
     Fp* eq = (Fp*)c->scratch(n * 4 + 16);
-    eq_evals_kernel<Fp><<<grid_for(c, n), 256, 0, c->stream>>>((const Fp*)point, k, eq);
+    chain_launch(c, eq_evals_kernel<Fp>, grid_for(c, n), 256, 0, (const Fp*)point, k, eq);
     ZKB_LAUNCHED(c);
     const u32* tabs[3] = {(const u32*)eq, w, nullptr};
     ScOpts o;
@@ -344,7 +344,7 @@ inline MatmulRec prove_matmul_succinct_base(zkb_ctx* c, TrState* tr, const u32* 
         sb.run(c, tr);
     }
     Fp* eq_r = (Fp*)c->scratch(m_pad * 4 + 16);
-    eq_evals_kernel<Fp><<<grid_for(c, m_pad), 256, 0, c->stream>>>((const Fp*)r_dev, R.log_m, eq_r);
+    chain_launch(c, eq_evals_kernel<Fp>, grid_for(c, m_pad), 256, 0, (const Fp*)r_dev, R.log_m, eq_r);
     ZKB_LAUNCHED(c);
     u32* w_partial = (u32*)c->scratch(n_pad * 4 + 16);
     {
@@ -391,7 +391,7 @@ inline HadamardRec prove_hadamard_ef(zkb_ctx* c, TrState* tr, const u32* a, cons
     WidenEqArgs w{};
     w.src[0] = a; w.dst[0] = aef; w.len[0] = len; w.src[1] = b; w.dst[1] = bef; w.len[1] = len; w.nsrc = 2;
     w.point = point; w.eq_out = eq; w.k = k;
-    widen_eq_kernel<<<grid_for(c, n), 256, 0, c->stream>>>(w);
+    chain_launch(c, widen_eq_kernel, grid_for(c, n), 256, 0, w);
     ZKB_LAUNCHED(c);
     const u32* tabs[3] = {(const u32*)eq, (const u32*)aef, (const u32*)bef};
     ScOpts o;
@@ -421,7 +421,7 @@ inline AddRec prove_add_ef(zkb_ctx* c, TrState* tr, const u32* a, const u32* b, 
     WidenEqArgs w{};
     w.src[0] = a; w.dst[0] = aef; w.len[0] = len; w.src[1] = b; w.dst[1] = bef; w.len[1] = len; w.nsrc = 2;
     w.point = point; w.eq_out = eq; w.k = k;
-    widen_eq_kernel<<<grid_for(c, n), 256, 0, c->stream>>>(w);
+    chain_launch(c, widen_eq_kernel, grid_for(c, n), 256, 0, w);
     ZKB_LAUNCHED(c);
     const u32* ta[3] = {(const u32*)eq, (const u32*)aef, nullptr};
     ScOpts oa;
@@ -451,7 +451,7 @@ inline HadamardRec prove_hadamard_base(zkb_ctx* c, TrState* tr, const u32* a, co
     size_t n = size_t(1) << k;
     R.root = commit_small(c, cvec, (u32)n, nullptr, (u32)n, tr);
     Fp* eq = (Fp*)c->scratch(n * 4 + 16);
-    eq_evals_kernel<Fp><<<grid_for(c, n), 256, 0, c->stream>>>((const Fp*)point, k, eq);
+    chain_launch(c, eq_evals_kernel<Fp>, grid_for(c, n), 256, 0, (const Fp*)point, k, eq);
     ZKB_LAUNCHED(c);
     const u32* tabs[3] = {(const u32*)eq, a, b};
     R.sc = sumcheck_enqueue(c, tr, ZKB_SC_TRIPLE, tabs, k);
@@ -474,7 +474,7 @@ inline AddRec prove_add_base(zkb_ctx* c, TrState* tr, const u32* a, const u32* b
     size_t n = size_t(1) << k;
     R.root = commit_small(c, cvec, (u32)n, nullptr, (u32)n, tr);
     Fp* eq = (Fp*)c->scratch(n * 4 + 16);
-    eq_evals_kernel<Fp><<<grid_for(c, n), 256, 0, c->stream>>>((const Fp*)point, k, eq);
+    chain_launch(c, eq_evals_kernel<Fp>, grid_for(c, n), 256, 0, (const Fp*)point, k, eq);
     ZKB_LAUNCHED(c);
     const u32* ta[3] = {(const u32*)eq, a, nullptr};
     R.sa = sumcheck_enqueue(c, tr, ZKB_SC_PRODUCT, ta, k);

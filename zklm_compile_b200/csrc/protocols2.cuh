@@ -63,7 +63,7 @@ inline RmsNormRec prove_rmsnorm_ef(zkb_ctx* c, TrState* tr, const u32* x, const 
         WidenEqArgs w{};
         w.src[0] = g; w.dst[0] = g_ef; w.len[0] = (u32)n; w.src[1] = gamma_pad; w.dst[1] = gamma_ef; w.len[1] = (u32)n;
         w.src[2] = x; w.dst[2] = x_ef; w.len[2] = (u32)n; w.nsrc = 3; w.point = gc; w.eq_out = eq; w.k = k;
-        widen_eq_kernel<<<grid_for(c, n), 256, 0, c->stream>>>(w);
+        chain_launch(c, widen_eq_kernel, grid_for(c, n), 256, 0, w);
         ZKB_LAUNCHED(c);
     }
     const u32* tgp[3] = {(const u32*)eq, (const u32*)g_ef, nullptr};
@@ -85,7 +85,7 @@ inline RmsNormRec prove_rmsnorm_ef(zkb_ctx* c, TrState* tr, const u32* x, const 
         WidenEqArgs w{};
         w.src[0] = y; w.dst[0] = h_ef; w.len[0] = (u32)n; w.nsrc = 1;
         w.point = (const Fe*)(c->rec_dev + R.sq_point); w.eq_out = eq2; w.k = k;
-        widen_eq_kernel<<<grid_for(c, n), 256, 0, c->stream>>>(w);
+        chain_launch(c, widen_eq_kernel, grid_for(c, n), 256, 0, w);
         ZKB_LAUNCHED(c);
     }
     const u32* ths[3] = {(const u32*)eq2, (const u32*)h_ef, (const u32*)h_ef};
@@ -155,7 +155,7 @@ inline RmsNormRec prove_rmsnorm_base(zkb_ctx* c, TrState* tr, const u32* x, cons
     R.gc_point = c->rec_alloc(k);
     { ScriptBuilder sb; sb.squeeze(c->rec_dev + R.gc_point, k); sb.run(c, tr); }
     Fp* eq = (Fp*)c->scratch(n * 4 + 16);
-    eq_evals_kernel<Fp><<<grid_for(c, n), 256, 0, c->stream>>>((const Fp*)(c->rec_dev + R.gc_point), k, eq);
+    chain_launch(c, eq_evals_kernel<Fp>, grid_for(c, n), 256, 0, (const Fp*)(c->rec_dev + R.gc_point), k, eq);
     ZKB_LAUNCHED(c);
     const u32* tgp[3] = {(const u32*)eq, g, nullptr};
     R.g_prod = sumcheck_enqueue(c, tr, ZKB_SC_PRODUCT, tgp, k);
@@ -168,7 +168,7 @@ inline RmsNormRec prove_rmsnorm_base(zkb_ctx* c, TrState* tr, const u32* x, cons
     R.sq_point = c->rec_alloc(k);
     { ScriptBuilder sb; sb.squeeze(c->rec_dev + R.sq_point, k); sb.run(c, tr); }
     Fp* eq2 = (Fp*)c->scratch(n * 4 + 16);
-    eq_evals_kernel<Fp><<<grid_for(c, n), 256, 0, c->stream>>>((const Fp*)(c->rec_dev + R.sq_point), k, eq2);
+    chain_launch(c, eq_evals_kernel<Fp>, grid_for(c, n), 256, 0, (const Fp*)(c->rec_dev + R.sq_point), k, eq2);
     ZKB_LAUNCHED(c);
     const u32* ths[3] = {(const u32*)eq2, y, y};
     R.h_sq = sumcheck_enqueue(c, tr, ZKB_SC_TRIPLE, ths, k);
@@ -256,7 +256,7 @@ inline LookupRec prove_lookup_ef(zkb_ctx* c, TrState* tr, const u32* table_out, 
         memcpy(pre + 23, &n64, 8);
         size_t max_chunks = ((size_t)(2 * n + 2) * 4 + 31 + 1023) / 1024 + 1;
         u32* cvs = (u32*)c->scratch(max_chunks * 32);
-        b3_commit_kernel<<<1, c->single_cta_threads(), 0, c->stream>>>(b3_prefix(pre, 31), cat, 2 * n + 2, nullptr, cvs, c->rec_dev + R.digest, nullptr);
+        chain_launch(c, b3_commit_kernel, 1, c->single_cta_threads(), 0, b3_prefix(pre, 31), cat, 2 * n + 2, nullptr, cvs, c->rec_dev + R.digest, nullptr);
         ZKB_LAUNCHED(c);
     }
     return R;
@@ -332,7 +332,7 @@ inline LookupRec prove_lookup_base(zkb_ctx* c, TrState* tr, const u32* table_out
         memcpy(pre + 23, &n64, 8);
         size_t max_chunks = ((size_t)(2 * n + 2) * 4 + 31 + 1023) / 1024 + 1;
         u32* cvs = (u32*)c->scratch(max_chunks * 32);
-        b3_commit_kernel<<<1, c->single_cta_threads(), 0, c->stream>>>(b3_prefix(pre, 31), cat, 2 * n + 2, nullptr, cvs, c->rec_dev + R.digest, nullptr);
+        chain_launch(c, b3_commit_kernel, 1, c->single_cta_threads(), 0, b3_prefix(pre, 31), cat, 2 * n + 2, nullptr, cvs, c->rec_dev + R.digest, nullptr);
         ZKB_LAUNCHED(c);
     }
     return R;

@@ -212,6 +212,7 @@ __device__ __forceinline__ void sc_hash_by_pair(u32* t, const ScIO& io, unsigned
 // ---- multi-CTA round launch ----------------------------------------------------------------
 template <int KIND, class SrcT, class ChalT, bool FOLD>
 __global__ void __launch_bounds__(256) sc_round_kernel(ScTables tb, size_t half, u32 round, ScIO io) {
+    pdl_small_prologue();
     typedef typename Sel<FOLD, ChalT, SrcT>::type AccT;
     constexpr int NACC = ScTraits<KIND>::NACC, WA = Width<AccT>::W, NW = NACC * WA;
     __shared__ u32 red[32 * 16];
@@ -290,6 +291,7 @@ __device__ __forceinline__ void sc_base_coef_accum(u64* acc, u32 fa, u32 fb, u32
 // the round message (the fused launch below folds two challenges at once from the base tables).
 template <class ChalT, bool FOLD, bool WRITE = true>
 __global__ void __launch_bounds__(256) sc_product_base_kernel(ScTables tb, size_t half, u32 round, ScIO io) {
+    pdl_small_prologue();
     constexpr int NACC = FOLD ? 9 : 3;
     __shared__ u32 red[32 * 16];
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
@@ -400,6 +402,7 @@ template <> struct LdVec<4> { static __device__ __forceinline__ void ld(const u3
 // whose message is produced (2); challenges of rounds round-2 and round-1 are read from io.chal.
 template <int VEC>
 __global__ void __launch_bounds__(256) sc_product_base_fold2_kernel(ScTables tb, size_t E, u32 round, ScIO io) {
+    pdl_small_prologue();
     __shared__ u32 red[32 * 16];
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     __shared__ bool is_last;
@@ -469,6 +472,7 @@ __global__ void __launch_bounds__(256) sc_product_base_fold2_kernel(ScTables tb,
 // a pair costs nine EF products, about 2600 issue slots of field reductions with the folds: 3292 us, not kept.)
 // `q` = a quarter of the tables' length, a multiple of four.
 __global__ void __launch_bounds__(256) sc_product_base_two_kernel(ScTables tb, size_t q, u32 round, ScIO io) {
+    pdl_small_prologue();
     __shared__ u32 red[32 * 16];
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     __shared__ bool is_last;
@@ -536,6 +540,7 @@ __device__ __forceinline__ void sc_post_squeezes(TrPair& tr, const ScIO& io, con
 template <int KIND, class SrcT, class ChalT>
 __global__ void __launch_bounds__(SC_TAIL_THREADS) sc_tail_kernel(ScTables tb, size_t size, u32 round, u32 num_vars,
                                                                   int pending, ScIO io) {
+    pdl_small_prologue();
     constexpr int NT = ScTraits<KIND>::NT, NACC = ScTraits<KIND>::NACC;
     constexpr int WC = Width<ChalT>::W, WS = Width<SrcT>::W;
     __shared__ u32 red[32 * 16];

@@ -124,6 +124,7 @@ __device__ __forceinline__ void pipe_worker_pass(const T* rf, const T* rg, T* wf
 template <class T>
 __global__ void __launch_bounds__(PIPE_THREADS) sc_tail_product_pipe_kernel(ScTables tb, size_t size, u32 round, u32 num_vars,
                                                                                int pending, ScIO io) {
+    pdl_small_prologue();
     constexpr int W = Width<T>::W, NW = PIPE_NW<T>;
     __shared__ u32 red[32 * 16];
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];

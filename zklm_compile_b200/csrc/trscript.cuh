@@ -76,6 +76,7 @@ struct TrScript {
 
 constexpr int TRSCRIPT_THREADS = 64;      // warp 0 advances the transcript, warp 1 prefetches and expands (see tr_absorb_stream_2w)
 __global__ void __launch_bounds__(TRSCRIPT_THREADS) tr_script_kernel(TrState* st, TrScript sc) {
+    pdl_small_prologue();
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     __shared__ u32 tile[2 * 512];
     __shared__ __align__(16) u32 kw[2 * 32 * SHA_KW_STRIDE];
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(TRSCRIPT_THREADS) tr_script_kernel(TrState* st
 // device-resident length (LogUp's number of active table entries).
 __global__ void __launch_bounds__(1024) b3_commit_kernel(B3Prefix pre, const u32* __restrict__ words, u32 n_words,
                                                          const u32* n_words_dev, u32* cvs_scratch, u32* root_out, TrState* absorb_into) {
+    pdl_small_prologue();
     __shared__ __align__(16) unsigned char trbuf[TR_SCRATCH_BYTES];
     if (n_words_dev) n_words = n_words_dev[0];
     b3_hash_block(pre, words, n_words, cvs_scratch);
