@@ -1,5 +1,5 @@
 // Device-resident Fiat-Shamir transcript: a SHA-256 stream that lives in global memory and is
-// advanced by one thread of whichever kernel finishes a protocol step, so challenges never
+// advanced by one thread, or by one warp with a second one beside it, of whichever kernel finishes a protocol step, so challenges never
 // travel to the host.  Mirrors the reference `Transcript`
 // (rust/zk_ml_prover/src/proving/sumcheck.rs:110-206):
 //   new(label)      stream = label bytes
