@@ -1,7 +1,8 @@
 /* A CUDA runtime without a GPU, for tests of the host code's stream order: memory is host memory, kernels do nothing, copies are
  * made at once, and every operation on a stream is counted.  Events carry what their stream was ordered after, so that
  * fake_unordered() can tell how many operations of other streams a stream (or the host) has not been made to wait for.
- * fake_fail_at(n) lets the n-th fallible call from then on return cudaErrorMemoryAllocation. */
+ * fake_fail_at(n) lets the n-th fallible call from then on return cudaErrorMemoryAllocation.  A capture records nothing, its
+ * operations count like others; it ends with an error while a stream is not joined.  fake_graph_flags(): of the last instantiation. */
 #include <cuda_runtime_api.h>
 #include <stdlib.h>
 #include <string.h>
@@ -18,6 +19,7 @@ static long calls, fail_at = -1;
 static dim3 cfg_grid, cfg_block;
 static size_t cfg_smem;
 static cudaStream_t cfg_stream;
+static long graph_flags = -1;
 
 static int id_of(cudaStream_t s) { return s ? s->id : 0; }
 static void op(cudaStream_t s) { int i = id_of(s); known[i].at[i] = ++done[i]; }
@@ -26,6 +28,7 @@ static cudaError_t fallible(void) { return calls++ == fail_at ? cudaErrorMemoryA
 #define FALLIBLE do { cudaError_t e_ = fallible(); if (e_) return e_; } while (0)
 
 long fake_calls(void) { return calls; }
+long fake_graph_flags(void) { return graph_flags; }
 void fake_fail_at(long n) { calls = 0; fail_at = n; }
 long fake_unordered(cudaStream_t s) {
     long n = 0;
@@ -53,6 +56,7 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, enum cudaMemcpyKin
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t st) { FALLIBLE; memset(d, v, n); op(st); return cudaSuccess; }
 cudaError_t cudaFuncSetAttribute(const void* f, enum cudaFuncAttribute a, int v) { (void)f; (void)a; (void)v; FALLIBLE; return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned f) { (void)f; FALLIBLE; streams[n_streams].id = n_streams; *s = &streams[n_streams++]; return cudaSuccess; }
+cudaError_t cudaStreamCreateWithPriority(cudaStream_t* s, unsigned f, int p) { (void)p; return cudaStreamCreateWithFlags(s, f); }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { (void)s; return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { merge(&host, &known[id_of(s)]); return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned f) { (void)f; FALLIBLE; merge(&known[id_of(s)], &e->c); return cudaSuccess; }
@@ -64,6 +68,16 @@ unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t m, struct CUstream_s
 cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* m, void* s) { *g = cfg_grid; *b = cfg_block; *m = cfg_smem; *(cudaStream_t*)s = cfg_stream; return cudaSuccess; }
 cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3 b, void** a, size_t m, cudaStream_t s) { (void)f; (void)g; (void)b; (void)a; (void)m; op(s); return cudaSuccess; }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** a) { (void)f; (void)a; FALLIBLE; op(c->stream); return cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t s, enum cudaStreamCaptureMode m) { (void)s; (void)m; FALLIBLE; return cudaSuccess; }
+cudaError_t cudaStreamEndCapture(cudaStream_t s, cudaGraph_t* g) {
+    FALLIBLE;
+    *g = fake_unordered(s) ? NULL : (cudaGraph_t)&graph_flags;
+    return *g ? cudaSuccess : cudaErrorStreamCaptureUnjoined;
+}
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t g, unsigned long long f) { FALLIBLE; *e = (cudaGraphExec_t)g; graph_flags = (long)f; return cudaSuccess; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t s) { (void)e; FALLIBLE; op(s); return cudaSuccess; }
+cudaError_t cudaGraphDestroy(cudaGraph_t g) { (void)g; return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) { (void)e; return cudaSuccess; }
 void** __cudaRegisterFatBinary(void* f) { static void* h; (void)f; return &h; }
 void __cudaRegisterFatBinaryEnd(void** h) { (void)h; }
 void __cudaUnregisterFatBinary(void** h) { (void)h; }

@@ -16,11 +16,12 @@ import ctypes as C
 import sys
 import numpy as np
 import zklm_compile_b200 as zk
-from zklm_compile_b200 import _lib, attention, pcs, tables
+from tests.util import rand_layer
+from zklm_compile_b200 import _lib, attention, pcs, qwen, tables
 from oracle import pyoracle as O
 
 fake = C.CDLL(None)
-fake.fake_calls.restype = fake.fake_unordered.restype = C.c_long
+fake.fake_calls.restype = fake.fake_unordered.restype = fake.fake_graph_flags.restype = C.c_long
 fake.fake_unordered.argtypes = [C.c_void_p]
 fake.fake_fail_at.argtypes = [C.c_long]
 ctx = zk.Context(0)
@@ -59,6 +60,18 @@ def attention_verify():
     assert status == 0
     return lambda tr: attention.verify_row_attention(blob, Q, V, H, S, D, tr)
 
+KEEP = []
+
+def layer(binding, graph=False):
+    silu, sigmoid = ctx.upload(tables.build_silu_table(1000)), ctx.upload(tables.build_sigmoid_table(1000))
+    cfg, weights, x = rand_layer(1, d_model=24, d_ff=40, heads=2, kv=1, d_head=8)
+    L = qwen.QwenLayer(ctx, cfg, weights, silu, sigmoid)
+    L.set_binding(binding)
+    L.use_graph(graph)
+    L.forward(x)
+    KEEP.append(L)                           # freeing one waits for the device
+    return lambda tr: L.prove(0, bytes(32))
+
 def in_order(what):
     left = fake.fake_unordered(main)
     assert left == 0, "%s: %d operations of the second stream are not joined" % (what, left)
@@ -77,6 +90,14 @@ if sys.argv[1] == "exhausted":
     ok = batch([1 << 14, 1 << 10])
     ok(tr)
     in_order("the call behind it")
+elif sys.argv[1] == "graph":
+    prove = layer(2, True)
+    for i in range(3):                       # launch by launch, captured, replayed
+        prove(None)
+        in_order("proof %d" % i)
+        assert KEEP[0].graph_state() == (1, 2, 2)[i], (i, KEEP[0].graph_state())
+    use_node_priority = 8
+    assert fake.fake_graph_flags() & use_node_priority, "a replay runs every kernel at the priority of the stream it is launched into"
 else:
     call = eval(sys.argv[1])
     tr = zk.Transcript(ctx, b"t")
@@ -117,6 +138,10 @@ def run(runtime, what):
 
 def test_batch_that_exhausts_the_record_buffer(runtime):
     run(runtime, "exhausted")
+
+
+def test_replays_of_a_layer_proof_keep_the_priorities_of_their_streams(runtime):
+    run(runtime, "graph")
 
 
 @pytest.mark.parametrize("call", ["basefold(5000)", "batch([1 << 14, 1 << 13, 1 << 13, 300, 7])", "basefold_verify(300)", "batch_verify([300, 70])",
