@@ -295,3 +295,52 @@ def test_qwen_model_shared_contexts_prove_in_waves_pcs_full():
         assert c.scratch_bytes == 0
     assert model.forward_and_prove(x) == exp[::-1]      # the arena grows again
     model.close()
+
+
+@pytest.mark.parametrize("mode,kind,shape,against_oracle", [(1, 0, dict(d_model=64, d_ff=96, heads=4, kv=2, d_head=16), True),
+                                                             (2, 0, dict(d_model=64, d_ff=96, heads=4, kv=2, d_head=16), True),
+                                                             (2, 1, dict(d_model=64, d_ff=96, heads=4, kv=2, d_head=16), True),
+                                                             (2, 0, dict(d_model=500, d_ff=1400, heads=4, kv=1, d_head=60), False),
+                                                             (2, 1, dict(d_model=300, d_ff=1900, heads=4, kv=4, d_head=64), False)])
+def test_replayed_layer_proofs_with_basefold_binding(ctx, mode, kind, shape, against_oracle):
+    """Two layers in two contexts, proved at the same time and six times each: launch by launch (twice where the arena came in pieces the
+    first time), captured, then replayed, with another input each time.  The expected bytes are the oracle's; for matrices of up to 2^20 coefficients of unequal sizes, where commitments are made
+    while the opening before them runs and rounds have launches of their own, those of a context that does everything in order."""
+    import hashlib
+    from zklm_compile_b200 import qwen as zq
+    from tests.util import load_qwen_golden, rand_layer
+    G = load_qwen_golden()
+    ih = hashlib.sha256(b"model-input").digest()
+    cfgs, weights, _ = zip(*(rand_layer(70 + i, **shape) for i in range(2)))
+    ctxs = [zk.Context(0) for _ in range(2)]
+    tables = [(c.upload(G["silu"]), c.upload(G["sigmoid"])) for c in ctxs + [ctx]]
+    layers = [zq.QwenLayer(c, cfgs[i], weights[i], *tables[i]) for i, c in enumerate(ctxs)]
+    plain = None if against_oracle else [zq.QwenLayer(ctx, cfgs[i], weights[i], *tables[2]) for i in range(2)]
+    for l in layers + (plain or []):
+        l.set_binding(mode, kind)
+    try:
+        ctx.set_option(ctx.OPT_BASEFOLD_IN_ORDER, 1)
+        for step in range(6):
+            x = rand_layer(90 + step, **shape)[2]
+            if step > 3:
+                assert [l.graph_state() for l in layers] == [2, 2]
+            for l in layers:
+                l.forward(x)
+            for i, l in enumerate(layers):
+                l.prove_begin(i, ih)
+            proofs = [l.prove_end() for l in layers]
+            for i in range(2):
+                if against_oracle:
+                    with O.features(mode, kind):
+                        want = O.qwen_layer_prove(cfgs[i], weights[i], x, G["silu"], G["sigmoid"], i, ih, verify=False)[1]
+                else:
+                    plain[i].use_graph(False)
+                    plain[i].forward(x)
+                    want = plain[i].prove(i, ih)
+                assert proofs[i] == want, (step, i)
+    finally:
+        ctx.set_option(ctx.OPT_BASEFOLD_IN_ORDER, 0)
+        for l in layers + (plain or []):
+            l.close()
+        for c in ctxs:
+            c.close()
