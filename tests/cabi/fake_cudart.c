@@ -2,7 +2,8 @@
  * made at once, and every operation on a stream is counted.  Events carry what their stream was ordered after, so that
  * fake_unordered() can tell how many operations of other streams a stream (or the host) has not been made to wait for.
  * fake_fail_at(n) lets the n-th fallible call from then on return cudaErrorMemoryAllocation.  A capture records nothing, its
- * operations count like others; it ends with an error while a stream is not joined.  fake_graph_flags(): of the last instantiation. */
+ * operations count like others; it ends with an error while a stream is not joined.  Memory is zero at first (from 32 MB on it comes
+ * from the system).  fake_graph_flags(): of the last instantiation. */
 #include <cuda_runtime_api.h>
 #include <stdlib.h>
 #include <string.h>
@@ -46,7 +47,7 @@ cudaError_t cudaGetDeviceProperties_v2(struct cudaDeviceProp* p, int d) { (void)
 cudaError_t cudaDeviceGetStreamPriorityRange(int* lo, int* hi) { *lo = 0; *hi = -5; return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t e) { return e ? "planted by the fake runtime" : "no error"; }
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
-cudaError_t cudaMalloc(void** p, size_t n) { FALLIBLE; *p = NULL; void* q = NULL; if (posix_memalign(&q, 256, n ? n : 1)) return cudaErrorMemoryAllocation; *p = q; return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) { FALLIBLE; *p = NULL; void* q = NULL; if (posix_memalign(&q, 256, n ? n : 1)) return cudaErrorMemoryAllocation; if (n < (32u << 20)) memset(q, 0, n); *p = q; return cudaSuccess; }
 cudaError_t cudaFree(void* p) { for (int i = 0; i < n_streams; i++) host.at[i] = done[i]; free(p); return cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned f) { (void)f; FALLIBLE; *p = calloc(n ? n : 1, 1); return *p ? cudaSuccess : cudaErrorMemoryAllocation; }
 cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }

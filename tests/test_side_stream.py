@@ -62,9 +62,9 @@ def attention_verify():
 
 KEEP = []
 
-def layer(binding, graph=False):
+def layer(binding, graph=False, d_model=24, d_ff=40, d_head=8):
     silu, sigmoid = ctx.upload(tables.build_silu_table(1000)), ctx.upload(tables.build_sigmoid_table(1000))
-    cfg, weights, x = rand_layer(1, d_model=24, d_ff=40, heads=2, kv=1, d_head=8)
+    cfg, weights, x = rand_layer(1, d_model=d_model, d_ff=d_ff, heads=2, kv=1, d_head=d_head)
     L = qwen.QwenLayer(ctx, cfg, weights, silu, sigmoid)
     L.set_binding(binding)
     L.use_graph(graph)
@@ -98,6 +98,17 @@ elif sys.argv[1] == "graph":
         assert KEEP[0].graph_state() == (1, 2, 2)[i], (i, KEEP[0].graph_state())
     use_node_priority = 8
     assert fake.fake_graph_flags() & use_node_priority, "a replay runs every kernel at the priority of the stream it is launched into"
+elif sys.argv[1] == "arena":
+    # Matrices of 2^22 coefficients, every one bound by an opening: 42 bytes a coefficient are in use at most (codeword and tree 20, those of
+    # the folds 20, values 2), and the first proof asks for them in pieces of 64 MB and more.
+    for in_order_option in (0, 1):
+        ctx = zk.Context(0)
+        KEEP.append(ctx)
+        ctx.set_option(ctx.OPT_BASEFOLD_IN_ORDER, in_order_option)
+        prove = layer(2, False, d_model=1024, d_ff=4096, d_head=128)
+        for _ in range(3):
+            prove(None)
+        assert ctx.scratch_bytes <= 64 << 22, ctx.scratch_bytes
 else:
     call = eval(sys.argv[1])
     tr = zk.Transcript(ctx, b"t")
@@ -119,6 +130,9 @@ else:
         in_order("the call behind it")
     assert refused > n // 2, (refused, n)
     print(n, refused)
+import os
+sys.stdout.flush()
+os._exit(0)                                  # nothing is freed: that waits for streams of contexts that are gone
 """
 
 
@@ -144,7 +158,11 @@ def test_replays_of_a_layer_proof_keep_the_priorities_of_their_streams(runtime):
     run(runtime, "graph")
 
 
+def test_commitments_ahead_take_no_more_memory_than_between_the_openings(runtime):
+    run(runtime, "arena")
+
+
 @pytest.mark.parametrize("call", ["basefold(5000)", "batch([1 << 14, 1 << 13, 1 << 13, 300, 7])", "basefold_verify(300)", "batch_verify([300, 70])",
-                                  "attention_prove()", "attention_verify()"])
+                                  "attention_prove()", "attention_verify()", "layer(1)", "layer(2)"])
 def test_any_failing_runtime_call(runtime, call):
     run(runtime, call)

@@ -439,11 +439,6 @@ inline u32 bf_chain_rounds(u32 round, u32 log_n) {
 
 // One half of a polynomial's codeword and its tree; nothing in it depends on the transcript.
 struct BfCommit { u32* cw = nullptr; uint4* tree = nullptr; };
-inline size_t bf_commit_bytes(u32 log_n) { return (size_t(4) << log_n) + 256 + mk_node_count(log_n) * 16 + 16; }
-inline BfCommit bf_commit_place(void* mem, u32 log_n) {
-    const size_t cw = ((size_t(4) << log_n) + 255) & ~size_t(255);
-    return BfCommit{(u32*)mem, (uint4*)((char*)mem + cw)};
-}
 inline void bf_commit_enqueue(zkb_ctx* c, CoefSrc src, u32 log_n, int kind, const BfTables& tb, BfCommit to) {
     c->prof_mark();
     bf_encode(c, src, log_n, tb, to.cw, false);
@@ -456,7 +451,7 @@ inline void bf_commit_enqueue(zkb_ctx* c, CoefSrc src, u32 log_n, int kind, cons
 
 // Enqueue commit + opening of the polynomial `src` (num_coeffs live coefficients, padded view of
 // 2^log_n) at the device-resident point.  The transcript first absorbs the commitment root.  `made`: the commitment, if it
-// has been made already.
+// has been made already; what is enqueued on the second stream behind this opening may then use its memory again.
 inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t num_coeffs, u32 log_n, const u32* point_dev, u32 n_point,
                                   int kind, const BfCommit* made = nullptr) {
     if (log_n < 1 || log_n > 28) throw ArgFail{ZKB_E_TOO_LARGE, "basefold: log_n out of range"};
@@ -471,11 +466,10 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
     // the transcript: they run ahead on a second stream, each round into buffers of its own, while the
     // context's stream runs the hash chain (root absorb, 24 query squeezes) and the path gathers behind them.
     const bool ahead = n_point >= log_n && !c->opt_bf_in_order;
-    const BfCommit commit = made ? *made : bf_commit_place(c->scratch(bf_commit_bytes(log_n)), log_n);
-    u32* cwA = commit.cw;
+    u32* cwA = made ? made->cw : (u32*)c->scratch(n_pad * 4);
     u32* cwB = ahead ? nullptr : (u32*)c->scratch(n_pad / 2 * 4);
     u32* eval = (u32*)c->scratch((n_pad / 2 + 4) * 4);
-    uint4* treeA = commit.tree;
+    uint4* treeA = made ? made->tree : (uint4*)c->scratch(mk_node_count(log_n) * 16 + 16);
     uint4* treeB = ahead ? nullptr : (uint4*)c->scratch(mk_node_count(log_n) * 16 + 16);
     u32* alpha = (u32*)c->scratch((log_n + 1) * 4);
     std::vector<u32*> cws{cwA};            // the folded codeword of each round: the first fold's is the codeword's half itself
@@ -487,7 +481,7 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
         }
     }
 
-    if (!made) bf_commit_enqueue(c, src, log_n, kind, tb, commit);
+    if (!made) bf_commit_enqueue(c, src, log_n, kind, tb, BfCommit{cwA, treeA});
     SideFork fork(c, ahead, log_n);
     pd.root_off = c->rec_alloc(4);
     bf_begin_kernel<<<1, 1, 0, c->stream>>>(tr, treeA + mk_node_count(log_n), point_dev, n_point, alpha, c->rec_dev + pd.root_off);
@@ -544,14 +538,28 @@ inline BfPending basefold_enqueue(zkb_ctx* c, TrState* tr, CoefSrc src, size_t n
         }
     }
     if (ahead) {
-        for (rounds.first = 0; rounds.first < log_n; rounds.first += rounds.count) {
-            rounds.count = bf_chain_rounds(rounds.first, log_n);
-            ZKB_CUDA(cudaStreamWaitEvent(fork.main, c->side_event(rounds.first + rounds.count - 1), 0));
+        // Only rounds 0 and 1 open paths of the commitment.  Where its memory is wanted again they are gathered on the second stream as
+        // soon as their positions are known, the others together behind the last round.
+        const u32 early = made ? (log_n < 2 ? log_n : 2) : 0;
+        bool gathered = early == 0;
+        for (u32 first = 0; first < log_n; first += rounds.count) {
+            rounds.first = first; rounds.count = bf_chain_rounds(first, log_n);
+            ZKB_CUDA(cudaStreamWaitEvent(fork.main, c->side_event(first + rounds.count - 1), 0));
             bf_launch_chain(c, rounds);
+            if (!gathered && first + rounds.count >= early) {
+                BfRounds r = rounds;
+                r.first = 0; r.count = early;
+                ZKB_CUDA(cudaEventRecord(c->side_event(log_n + 1), fork.main));
+                ZKB_CUDA(cudaStreamWaitEvent(fork.side, c->side_event(log_n + 1), 0));
+                c->stream = fork.side;
+                bf_launch_gather(c, r);
+                c->stream = fork.main;
+                gathered = true;
+            }
         }
-        fork.joined();
-        rounds.first = 0; rounds.count = log_n;
-        bf_launch_gather(c, rounds);
+        if (early) fork.join(); else fork.joined();
+        rounds.first = early; rounds.count = log_n - early;
+        if (rounds.count) bf_launch_gather(c, rounds);
     }
     pd.final_off = c->rec_alloc(1);
     ZKB_CUDA(cudaMemcpyAsync(c->rec_dev + pd.final_off, eval, 4, cudaMemcpyDeviceToDevice, c->stream));

@@ -114,9 +114,10 @@ struct MatmulRec {
 };
 // The commitments of a sequence of openings, made ahead of the transcript on the second stream: while the hash chain of one opening and
 // of what lies between it and the next one runs (about 1.5 ms on one SM), the rest of the GPU encodes the next matrix and builds its
-// tree.  Two places take turns; the next commitment but one waits until the opening of the one before it is through with its place.
+// tree.  They take turns in one place: an opening is through with its commitment when the paths of its first two rounds are out, before
+// most of its chain has run, so this needs no more memory than committing between the openings.
 // Measured on B200, a layer of the 9B shape with all eight matrices bound, one after the other in a graph -> like this, the folds ahead
-// of the chain in the graph too: 51.1 -> 43.5 ms (encoding, trees and folds are 26 ms of the GPU, the hash chain 19 ms alone).
+// of the chain in the graph too: 51.1 -> 41.1 ms (encoding, trees and folds are 26 ms of the GPU, the hash chain 19 ms alone).
 struct BfAhead {
     struct Item { CoefSrc src; u32 log_n; };
     zkb_ctx* const c;
@@ -129,21 +130,22 @@ struct BfAhead {
         const u32 log_cols = log2_ceil_u(n);
         items.push_back(Item{CoefSrc{W, m, n, log_cols}, log2_ceil_u(m) + log_cols});
     }
-    // All matrices are known: places, and the first commitment behind what the context's stream holds.
+    // All matrices are known: the place, and the first commitment behind what the context's stream holds.
     void start() {
         if (c->opt_bf_in_order || items.empty()) return;
         if (kind == NODE_AES_MMO) aes_tables_upload();
+        u32 longest = 0;
         for (auto& it : items) {
             if (it.log_n < 1 || it.log_n > 28) return;            // the opening itself reports it
             bf_tables(c, it.log_n);
+            longest = std::max(longest, it.log_n);
         }
-        size_t bytes[2] = {0, 0};
-        for (size_t i = 0; i < items.size(); i++) bytes[i & 1] = std::max(bytes[i & 1], bf_commit_bytes(items[i].log_n));
-        for (int p = 0; p < 2; p++) if (bytes[p]) place[p] = c->scratch(bytes[p]);
+        place = BfCommit{(u32*)c->scratch(size_t(4) << longest), (uint4*)c->scratch(mk_node_count(longest) * 16 + 16)};
         // from here to done() the context's stream is the lifted one
-        const cudaStream_t up = c->lifted_stream();
-        ZKB_CUDA(cudaEventRecord(c->side_event(EVENTS + 4), base));
-        ZKB_CUDA(cudaStreamWaitEvent(up, c->side_event(EVENTS + 4), 0));
+        const cudaStream_t up = c->lifted_stream(), side = c->side_stream();
+        ZKB_CUDA(cudaEventRecord(c->side_event(JOIN), base));
+        ZKB_CUDA(cudaStreamWaitEvent(up, c->side_event(JOIN), 0));
+        ZKB_CUDA(cudaStreamWaitEvent(side, c->side_event(JOIN), 0));
         on = true;
         c->stream = up;
         make();
@@ -151,22 +153,17 @@ struct BfAhead {
     // The commitment of the next opening, for the context's stream from here on; null when none was made.
     const BfCommit* take() {
         if (!on) return nullptr;
-        ZKB_CUDA(cudaStreamWaitEvent(c->stream, ready(used), 0));
-        current = bf_commit_place(place[used & 1], items[used].log_n);
-        return &current;
+        ZKB_CUDA(cudaStreamWaitEvent(c->stream, c->side_event(READY), 0));
+        return &place;
     }
-    // That opening has been enqueued: its folds are on the second stream, the commitment after it goes behind them.
-    void opened() {
-        if (!on) return;
-        ZKB_CUDA(cudaEventRecord(freed(used), c->stream));
-        used++;
-        if (made < items.size()) make();
-    }
+    // That opening has been enqueued: the second stream holds its folds and the gather of its first paths, the commitment after it goes
+    // behind them.
+    void opened() { if (on && made < items.size()) make(); }
     // The context's own stream goes on behind all of it.
     void done() {
         if (!on) return;
-        ZKB_CUDA(cudaEventRecord(c->side_event(EVENTS + 4), c->stream));
-        ZKB_CUDA(cudaStreamWaitEvent(base, c->side_event(EVENTS + 4), 0));
+        ZKB_CUDA(cudaEventRecord(c->side_event(JOIN), c->stream));
+        ZKB_CUDA(cudaStreamWaitEvent(base, c->side_event(JOIN), 0));
         c->stream = base;
         on = false;
     }
@@ -176,30 +173,23 @@ struct BfAhead {
         const cudaStream_t from[2] = {c->side, c->stream};
         c->stream = base;
         for (int i = 0; i < 2; i++)
-            if (cudaEventRecord(c->side_event(EVENTS + 4), from[i]) != cudaSuccess || cudaStreamWaitEvent(base, c->side_event(EVENTS + 4), 0) != cudaSuccess)
+            if (cudaEventRecord(c->side_event(JOIN), from[i]) != cudaSuccess || cudaStreamWaitEvent(base, c->side_event(JOIN), 0) != cudaSuccess)
                 cudaStreamSynchronize(from[i]);
     }
 
 private:
-    static constexpr size_t EVENTS = 40;          // behind those of an opening's rounds
+    static constexpr size_t READY = 40, JOIN = 41;          // events, behind those of an opening's rounds
     const cudaStream_t base;
-    void* place[2] = {nullptr, nullptr};
-    BfCommit current;
-    size_t made = 0, used = 0;
+    BfCommit place;
+    size_t made = 0;
     bool on = false;
-    cudaEvent_t ready(size_t i) { return c->side_event(EVENTS + (i & 1)); }
-    cudaEvent_t freed(size_t i) { return c->side_event(EVENTS + 2 + (i & 1)); }
     void make() {
-        const cudaStream_t main = c->stream, side = c->side_stream();
         const Item& it = items[made];
-        // the first one waits for what the stream holds, the third and later ones for the opening that used the place before
-        if (made == 0) ZKB_CUDA(cudaEventRecord(freed(0), main));
-        if (made != 1) ZKB_CUDA(cudaStreamWaitEvent(side, freed(made), 0));
         made++;
-        struct Restore { zkb_ctx* c; cudaStream_t s; ~Restore() { c->stream = s; } } restore{c, main};
-        c->stream = side;
-        bf_commit_enqueue(c, it.src, it.log_n, kind, bf_tables(c, it.log_n), bf_commit_place(place[(made - 1) & 1], it.log_n));
-        ZKB_CUDA(cudaEventRecord(ready(made - 1), side));
+        struct Restore { zkb_ctx* c; cudaStream_t s; ~Restore() { c->stream = s; } } restore{c, c->stream};
+        c->stream = c->side_stream();
+        bf_commit_enqueue(c, it.src, it.log_n, kind, bf_tables(c, it.log_n), place);
+        ZKB_CUDA(cudaEventRecord(c->side_event(READY), c->stream));
     }
 };
 
@@ -253,8 +243,9 @@ inline MatmulRec prove_matmul_succinct_ef(zkb_ctx* c, TrState* tr, const u32* W,
         CoefSrc src = bind == BIND_PCS_FULL ? CoefSrc{W, m, n, R.log_n} : CoefSrc{(const u32*)w_partial, 1, (u32)(4 * n_pad), R.log_n + 2};
         const u32 bf_log = bind == BIND_PCS_FULL ? R.log_m + R.log_n : R.log_n + 2;
         const size_t num_coeffs = bind == BIND_PCS_FULL ? (size_t)m * n : 4 * n_pad;
-        // codeword, trees and evaluation buffer (about 60 bytes per coefficient) are dead once the opening is
-        // enqueued: everything the proof keeps goes to the record, so the next protocol step reuses the memory
+        // folded codewords, their trees and the evaluation buffer (22 bytes per padded coefficient), and codeword and tree themselves (20) where
+        // they were not made ahead, are dead once the opening is enqueued: everything the proof keeps goes to the record, so the next
+        // protocol step reuses the memory
         const auto mark = c->scratch_mark();
         u32* bf_point = (u32*)c->scratch((bf_log + 1) * 4);
         ScriptBuilder sb;
