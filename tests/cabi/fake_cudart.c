@@ -25,7 +25,8 @@ static long graph_flags = -1;
 static int id_of(cudaStream_t s) { return s ? s->id : 0; }
 static void op(cudaStream_t s) { int i = id_of(s); known[i].at[i] = ++done[i]; }
 static void merge(Clock* a, const Clock* b) { for (int i = 0; i < MAX_STREAMS; i++) if (b->at[i] > a->at[i]) a->at[i] = b->at[i]; }
-static cudaError_t fallible(void) { return calls++ == fail_at ? cudaErrorMemoryAllocation : cudaSuccess; }
+static cudaError_t last_error;                          /* of this thread's calls, until it is asked for */
+static cudaError_t fallible(void) { return calls++ == fail_at ? (last_error = cudaErrorMemoryAllocation) : cudaSuccess; }
 #define FALLIBLE do { cudaError_t e_ = fallible(); if (e_) return e_; } while (0)
 
 long fake_calls(void) { return calls; }
@@ -46,7 +47,7 @@ cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaGetDeviceProperties_v2(struct cudaDeviceProp* p, int d) { (void)d; memset(p, 0, sizeof *p); p->major = 10; p->multiProcessorCount = 148; return cudaSuccess; }
 cudaError_t cudaDeviceGetStreamPriorityRange(int* lo, int* hi) { *lo = 0; *hi = -5; return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t e) { return e ? "planted by the fake runtime" : "no error"; }
-cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+cudaError_t cudaGetLastError(void) { cudaError_t e = last_error; last_error = cudaSuccess; return e; }
 cudaError_t cudaMalloc(void** p, size_t n) { FALLIBLE; *p = NULL; void* q = NULL; if (posix_memalign(&q, 256, n ? n : 1)) return cudaErrorMemoryAllocation; if (n < (32u << 20)) memset(q, 0, n); *p = q; return cudaSuccess; }
 cudaError_t cudaFree(void* p) { for (int i = 0; i < n_streams; i++) host.at[i] = done[i]; free(p); return cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned f) { (void)f; FALLIBLE; *p = calloc(n ? n : 1, 1); return *p ? cudaSuccess : cudaErrorMemoryAllocation; }

@@ -13,11 +13,15 @@ namespace zkb {
 
 struct CudaFail { std::string msg; };
 
+// A failure is reported once: the runtime keeps it for the thread's next cudaGetLastError, which would be the one at the end of a later
+// call that went well.
 #define ZKB_CUDA(expr)                                                                          \
     do {                                                                                        \
         cudaError_t _e = (expr);                                                                \
-        if (_e != cudaSuccess)                                                                  \
+        if (_e != cudaSuccess) {                                                                \
+            cudaGetLastError();                                                                 \
             throw ::zkb::CudaFail{std::string(#expr) + ": " + cudaGetErrorString(_e)};          \
+        }                                                                                       \
     } while (0)
 
 struct ArgFail { int32_t code; std::string msg; };
@@ -297,7 +301,10 @@ struct SideFork {
     void joined() { open = false; }      // the caller's own events have made `main` wait for all of it
     ~SideFork() {
         c->stream = main;
-        if (open && (cudaEventRecord(ev, side) != cudaSuccess || cudaStreamWaitEvent(main, ev, 0) != cudaSuccess)) cudaStreamSynchronize(side);
+        if (open && (cudaEventRecord(ev, side) != cudaSuccess || cudaStreamWaitEvent(main, ev, 0) != cudaSuccess)) {
+            cudaStreamSynchronize(side);
+            cudaGetLastError();
+        }
     }
 
 private:

@@ -173,8 +173,10 @@ struct BfAhead {
         const cudaStream_t from[2] = {c->side, c->stream};
         c->stream = base;
         for (int i = 0; i < 2; i++)
-            if (cudaEventRecord(c->side_event(JOIN), from[i]) != cudaSuccess || cudaStreamWaitEvent(base, c->side_event(JOIN), 0) != cudaSuccess)
+            if (cudaEventRecord(c->side_event(JOIN), from[i]) != cudaSuccess || cudaStreamWaitEvent(base, c->side_event(JOIN), 0) != cudaSuccess) {
                 cudaStreamSynchronize(from[i]);
+                cudaGetLastError();
+            }
     }
 
 private:

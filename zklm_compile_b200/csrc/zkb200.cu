@@ -467,6 +467,11 @@ std::mutex g_noalloc_mu;
 void set_err(char* err, size_t cap, const std::string& msg) {
     if (err && cap) { size_t n = msg.size() < cap - 1 ? msg.size() : cap - 1; memcpy(err, msg.data(), n); err[n] = 0; }
 }
+int32_t cuda_err(char* err, size_t cap, const char* what, cudaError_t e) {
+    set_err(err, cap, std::string(what) + cudaGetErrorString(e));
+    cudaGetLastError();                    // reported here, not by the thread's next call (see ZKB_CUDA)
+    return ZKB_E_CUDA;
+}
 }  // namespace
 
 extern "C" int32_t zkb_fold_eq_matvec_ef_noalloc(const uint32_t* W_dev, size_t m, size_t n, const uint32_t* eq_dev, uint32_t* out_dev,
@@ -484,7 +489,7 @@ extern "C" int32_t zkb_fold_eq_matvec_ef_noalloc(const uint32_t* W_dev, size_t m
     }
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess || dev < 0 || dev >= 64) { set_err(err, err_cap, std::string("cudaGetDevice: ") + cudaGetErrorString(e)); return ZKB_E_CUDA; }
+    if (e != cudaSuccess || dev < 0 || dev >= 64) return cuda_err(err, err_cap, "cudaGetDevice: ", e);
     NoallocDev& D = g_noalloc_dev[dev];
     {   // first call on this device: resolve the device address of the scratch array (the name
         // itself is only a host-side handle) with this device current
@@ -492,17 +497,17 @@ extern "C" int32_t zkb_fold_eq_matvec_ef_noalloc(const uint32_t* W_dev, size_t m
         if (!D.ready) {
             unsigned long long* p = nullptr;
             e = cudaGetSymbolAddress((void**)&p, g_noalloc_fold_acc);
-            if (e != cudaSuccess || !p) { set_err(err, err_cap, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e)); return ZKB_E_CUDA; }
+            if (e != cudaSuccess || !p) return cuda_err(err, err_cap, "cudaGetSymbolAddress: ", e);
             int sms = 0;
             e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            if (e != cudaSuccess || sms <= 0) { set_err(err, err_cap, std::string("cudaDeviceGetAttribute: ") + cudaGetErrorString(e)); return ZKB_E_CUDA; }
+            if (e != cudaSuccess || sms <= 0) return cuda_err(err, err_cap, "cudaDeviceGetAttribute: ", e);
             D.acc = p; D.sm_count = sms; D.ready = true;
         }
     }
     cudaStream_t s = (cudaStream_t)stream;
     // the array keeps whatever the previous call left: the accumulators must start at zero
     e = cudaMemsetAsync(D.acc, 0, n_pad * 4 * sizeof(unsigned long long), s);
-    if (e != cudaSuccess) { set_err(err, err_cap, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e)); return ZKB_E_CUDA; }
+    if (e != cudaSuccess) return cuda_err(err, err_cap, "cudaMemsetAsync: ", e);
     size_t rows_per = 0;
     dim3 grid = fold_launch_dims(D.sm_count, m, n, &rows_per);
     fold_eq_matvec_kernel<4, true><<<fold_grid(grid, D.sm_count, false), FOLD_THREADS, 0, s>>>(W_dev, m, n, eq_dev, rows_per, D.acc, nullptr);
@@ -511,6 +516,6 @@ extern "C" int32_t zkb_fold_eq_matvec_ef_noalloc(const uint32_t* W_dev, size_t m
     if (fin_grid > D.sm_count * 8) fin_grid = D.sm_count * 8;
     fold_finalize_kernel<4><<<fin_grid, 256, 0, s>>>(D.acc, n, n_pad, out_dev);
     e = cudaGetLastError();
-    if (e != cudaSuccess) { set_err(err, err_cap, std::string("kernel launch: ") + cudaGetErrorString(e)); return ZKB_E_CUDA; }
+    if (e != cudaSuccess) return cuda_err(err, err_cap, "kernel launch: ", e);
     return ZKB_OK;
 }
