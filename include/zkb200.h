@@ -189,7 +189,7 @@ int32_t zkb_basefold_batch_verify_opening(zkb_ctx* ctx, zkb_transcript* tr, cons
  * [, num_kv_heads], seq_len, d_head and then every row's scores and outputs - all of them in the proof - into its own transcript, as
  * attention.rs:140-143 and 254-265 do.  That stream is 4 * rows * (seq_len + d_head) bytes of strictly serial SHA-256, which a CPU core
  * with SHA instructions hashes about twenty times faster than one GPU thread (16 ms for the 1536 rows of a 12 x 128 x 64 call, the rows
- * themselves 1.1 ms): with tr the calling thread absorbs streams of 1024 words and more, and puts the state back in stream order. */
+ * themselves 1.1 ms): with tr the calling thread absorbs streams of 2560 words and more, and puts the state back in stream order. */
 int32_t zkb_row_attention_forward(zkb_ctx* ctx, const uint32_t* q, const uint32_t* k, const uint32_t* v, size_t num_heads, size_t seq_len,
                                   size_t d_head, const uint32_t* table_out, size_t n_table, int32_t on_device, uint32_t* out);
 int32_t zkb_prove_row_attention(zkb_ctx* ctx, zkb_transcript* tr, const uint32_t* q, const uint32_t* k, const uint32_t* v, size_t num_heads,

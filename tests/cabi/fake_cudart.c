@@ -16,7 +16,7 @@ static struct CUstream_st streams[MAX_STREAMS];
 static int n_streams = 1;                               /* 0: the default stream */
 static unsigned long long done[MAX_STREAMS];            /* operations enqueued so far */
 static Clock known[MAX_STREAMS], host;
-static long calls, fail_at = -1;
+static long calls, fail_at = -1, waits;
 static dim3 cfg_grid, cfg_block;
 static size_t cfg_smem;
 static cudaStream_t cfg_stream;
@@ -30,6 +30,7 @@ static cudaError_t fallible(void) { return calls++ == fail_at ? (last_error = cu
 #define FALLIBLE do { cudaError_t e_ = fallible(); if (e_) return e_; } while (0)
 
 long fake_calls(void) { return calls; }
+long fake_waits(void) { return waits; }                 /* of the host for a stream */
 long fake_graph_flags(void) { return graph_flags; }
 void fake_fail_at(long n) { calls = 0; fail_at = n; }
 long fake_unordered(cudaStream_t s) {
@@ -60,7 +61,7 @@ cudaError_t cudaFuncSetAttribute(const void* f, enum cudaFuncAttribute a, int v)
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned f) { (void)f; FALLIBLE; streams[n_streams].id = n_streams; *s = &streams[n_streams++]; return cudaSuccess; }
 cudaError_t cudaStreamCreateWithPriority(cudaStream_t* s, unsigned f, int p) { (void)p; return cudaStreamCreateWithFlags(s, f); }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { (void)s; return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t s) { merge(&host, &known[id_of(s)]); return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { waits++; merge(&host, &known[id_of(s)]); return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned f) { (void)f; FALLIBLE; merge(&known[id_of(s)], &e->c); return cudaSuccess; }
 cudaError_t cudaEventCreate(cudaEvent_t* e) { FALLIBLE; *e = calloc(1, sizeof **e); return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned f) { (void)f; return cudaEventCreate(e); }

@@ -38,9 +38,10 @@ def test_tails_match_oracle(ctx, option, kind, threads):
         ctx.set_option(getattr(ctx, option), 0)
 
 
-@pytest.mark.parametrize("heads,seq,d", [(1, 31, 2), (2, 16, 16), (3, 21, 17)])
+@pytest.mark.parametrize("heads,seq,d", [(1, 31, 2), (2, 16, 16), (3, 21, 17), (11, 8, 21), (2, 32, 8), (3, 23, 17)])
 def test_attention_transcript_at_the_host_absorb_line(ctx, heads, seq, d):
-    """Streams of 1023, 1024 and 2394 words: the caller's transcript absorbs them on the device below 1024 words, on the host from there on."""
+    """Streams of 1023, 1024, 2394, 2552, 2560 and 2760 words: the caller's transcript absorbs them on the device below 2560 words, on the host
+    from there on."""
     from zklm_compile_b200 import attention, tables
     rng = np.random.default_rng(seq)
     q, k = (np.mod(rng.integers(-1, 2, heads * seq * d), P).astype(np.uint32) for _ in range(2))

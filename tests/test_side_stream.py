@@ -21,7 +21,7 @@ from zklm_compile_b200 import _lib, attention, pcs, qwen, tables
 from oracle import pyoracle as O
 
 fake = C.CDLL(None)
-fake.fake_calls.restype = fake.fake_unordered.restype = fake.fake_graph_flags.restype = C.c_long
+fake.fake_calls.restype = fake.fake_waits.restype = fake.fake_unordered.restype = fake.fake_graph_flags.restype = C.c_long
 fake.fake_unordered.argtypes = [C.c_void_p]
 fake.fake_fail_at.argtypes = [C.c_long]
 ctx = zk.Context(0)
@@ -49,13 +49,14 @@ def batch_verify(sizes):
     blob = batch(sizes)(zk.Transcript(ctx, b"p"))
     return lambda tr: pcs.basefold_batch_verify_opening(ctx, tr, blob)
 
-H, S, D = 2, 5, 8
-Q, V, T = np.ones(H * S * D, np.uint32), poly(H * S * D), tables.build_exp_table(100)
+T = tables.build_exp_table(100)
 
-def attention_prove():
+def attention_prove(H=2, S=5, D=8):
+    Q, V = np.ones(H * S * D, np.uint32), poly(H * S * D)
     return lambda tr: attention.prove_row_attention(Q, Q, V, H, S, D, T, tr)
 
-def attention_verify():
+def attention_verify(H=2, S=5, D=8):
+    Q, V = np.ones(H * S * D, np.uint32), poly(H * S * D)
     blob, status = O.prove_row_attention(O.Transcript(b"p"), Q, Q, V, H, S, D, T)     # a proof of zeros would be turned away before any launch
     assert status == 0
     return lambda tr: attention.verify_row_attention(blob, Q, V, H, S, D, tr)
@@ -98,6 +99,17 @@ elif sys.argv[1] == "graph":
         assert KEEP[0].graph_state() == (1, 2, 2)[i], (i, KEEP[0].graph_state())
     use_node_priority = 8
     assert fake.fake_graph_flags() & use_node_priority, "a replay runs every kernel at the priority of the stream it is launched into"
+elif sys.argv[1] == "waits":
+    tr = zk.Transcript(ctx, b"t")
+    for make in (attention_prove, attention_verify):
+        waits = []
+        for shape in ((2, 5, 8), (1, 32, 32), (11, 8, 21), (2, 32, 8), (3, 23, 17)):      # 130, 2048, 2552, 2560, 2760 words
+            call = make(*shape)
+            call(tr)
+            before = fake.fake_waits()
+            call(tr)
+            waits.append(fake.fake_waits() - before)
+        assert waits == [waits[0]] * 3 + [waits[0] + 1] * 2, waits
 elif sys.argv[1] == "arena":
     # Matrices of 2^22 coefficients, every one bound by an opening: 42 bytes a coefficient are in use at most (codeword and tree 20, those of
     # the folds 20, values 2), and the first proof asks for them in pieces of 64 MB and more.
@@ -162,7 +174,11 @@ def test_commitments_ahead_take_no_more_memory_than_between_the_openings(runtime
     run(runtime, "arena")
 
 
+def test_short_streams_of_row_attention_do_not_make_the_host_wait(runtime):
+    run(runtime, "waits")
+
+
 @pytest.mark.parametrize("call", ["basefold(5000)", "batch([1 << 14, 1 << 13, 1 << 13, 300, 7])", "basefold_verify(300)", "batch_verify([300, 70])",
-                                  "attention_prove()", "attention_verify()", "layer(1)", "layer(2)"])
+                                  "attention_prove()", "attention_verify()", "attention_prove(2, 32, 32)", "attention_verify(2, 32, 32)", "layer(1)", "layer(2)"])
 def test_any_failing_runtime_call(runtime, call):
     run(runtime, call)

@@ -102,9 +102,11 @@ inline void tr_absorb_host(TrState& t, const void* bytes, size_t n) {
 
 // A long absorb of a caller's transcript on the host: begin() behind whatever advances the transcript, finish() once the words are here
 // and the context's stream, on which begin() was enqueued, has been waited for.
-// From HOST_ABSORB_MIN words on: below (64 blocks), the device's 0.87 us a block is not much more than the wait and the two copies.
-// Measured on B200, device -> host: checking 1232 attention rows with a stream of 15 785 blocks 14.96 -> 2.06 ms.
-constexpr size_t HOST_ABSORB_MIN = 1024;
+// From HOST_ABSORB_MIN words on: on the device such a stream takes about as long as the wait and the two copies (and row proofs of that many
+// words as long as either).  Measured on B200, device / host, us: a proof of 1280 words 348 / 362, of 1920 356 / 364, of 2448 376 / 382, of
+// 2560 373 / 369, of 2880 396 / 372, of 4096 470 / 386; checks and op lists of such proofs cross there too.  Checking 1232 attention rows with
+// a stream of 15 785 blocks 14.96 -> 2.06 ms.
+constexpr size_t HOST_ABSORB_MIN = 2560;
 struct HostAbsorb {
     zkb_ctx* const c;
     TrState* const dev;
