@@ -82,7 +82,8 @@ uint64_t zkb_ctx_scratch_bytes(const zkb_ctx* ctx);
  * ZKB_OPT_FOLD2_VEC: pair indices per thread (1, 2 or 4) of that two-challenge pass.
  * ZKB_OPT_BASEFOLD_IN_ORDER: nonzero = a Basefold opening runs fold, tree and transcript step of
  * each round one after another on the context's stream (normally the folds and trees of all rounds
- * whose challenge is a coordinate of the point run ahead on a second stream).
+ * whose challenge is a coordinate of the point run ahead on a second stream, and a layer proof that binds every matrix by
+ * an opening commits to the next matrix there).
  * ZKB_OPT_MATVEC_PREFETCH_ROWS: 0..8, rows per CTA that a forward matvec prefetches into L2 before it
  * waits for its input vector (default 2; 8 is the CTA's whole first pass; here 0 is a value, not "default").
  * ZKB_OPT_MATVEC_RING: nonzero = forward matvecs whose rows are a multiple of 16 bytes (at most 64 KB)

@@ -427,10 +427,12 @@ inline void bf_launch_chain(zkb_ctx* c, const BfRounds& a) {
 }
 // How many rounds the chain launch that starts at `round` takes when the trees run ahead on another stream: one while the
 // folded codewords are long (the next tree is still being built when this round's positions are known), then four,
-// then all the rest.  The line is where a fold and its tree take less than the chain's 30 us a round, so that from there on the
-// trees run away from the chain; measured on B200 alone on one stream, blake3 / AES: 2^20 values 71 / 82 us, 2^19 51 / 67, 2^18 37 / 48,
-// 2^17 29 / 39, 2^15 27 / 37, 2^10 16 / 24.  Two rounds later than at 46 us a round (16 below instead of 18): openings of 2^24
-// coefficients 2784 -> 2748 us, of 2^20 with AES nodes 1455 -> 1404, a batch of seven 2203 -> 2163; two rounds in the first group instead of four: 2820.
+// then all the rest.  With blake3 nodes the line is where a fold and its tree take less than the chain's 30 us a round, so that from there
+// on the trees run away from the chain: measured on B200 alone on one stream, blake3 / AES: 2^20 values 71 / 82 us, 2^19 51 / 67, 2^18 37 / 48,
+// 2^17 29 / 39, 2^15 27 / 37, 2^10 16 / 24.  AES trees of these sizes stay behind the chain, whose first launch of four rounds then waits for
+// them; the line is the same because it measured best there too: 16 below instead of 18 (the line when a round took 46 us), openings of 2^24
+// coefficients 2784 -> 2748 us, of 2^20 with AES nodes 1455 -> 1404, a batch of seven with AES nodes 2203 -> 2163; two rounds in the first
+// group instead of four: 2820.
 inline u32 bf_chain_rounds(u32 round, u32 log_n) {
     const u32 long_rounds = log_n > 16 ? log_n - 16 : 0;
     const u32 n = round < long_rounds ? 1 : (round == long_rounds ? 4 : log_n);

@@ -150,8 +150,6 @@ struct zkb_ctx {
     int opt_shared_sm = 0;               // 0: hash-chain kernels reserve 200 KB of shared memory, 1: none, 16 .. 200: that many KB
     bool opt_mv_ring = false;            // forward matvec: the bulk-copy ring kernel instead of the register-staged one
     int opt_mv_prefetch = 2;             // rows per CTA whose lines a forward matvec prefetches into L2 before it waits for its input (0 .. 8 measured: 2 is best)
-    // Second stream for work that does not depend on the transcript (the fold / tree chain of a Basefold
-    // opening), joined to `stream` through events; created on first use.
     // Page-locked staging for results that are larger than the record buffer; grows, freed with the context.
     void* stage = nullptr;
     size_t stage_cap = 0;
@@ -170,6 +168,8 @@ struct zkb_ctx {
         if (!tr_host) ZKB_CUDA(cudaHostAlloc(&tr_host, sizeof(zkb::TrState), cudaHostAllocDefault));
         return tr_host;
     }
+    // Second stream for work that does not depend on the transcript (the fold / tree chain of a Basefold
+    // opening), joined to `stream` through events; created on first use.
     cudaStream_t side = nullptr;
     std::vector<cudaEvent_t> side_ev;
     cudaStream_t side_stream() {
@@ -177,7 +177,8 @@ struct zkb_ctx {
         return side;
     }
     // A stream one priority above the second stream's, for a hash chain that runs beside wide kernels: at equal priority all blocks of
-    // the wide kernel that came first are placed before the chain's next one-block launch.
+    // the wide kernel that came first are placed before the chain's next one-block launch.  Captured graphs keep it (see where they are
+    // instantiated).
     cudaStream_t lifted = nullptr;
     cudaStream_t lifted_stream() {
         if (!lifted) {

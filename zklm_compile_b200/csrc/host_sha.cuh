@@ -1,7 +1,7 @@
 // SHA-256 over bytes that are in host memory anyway, by the calling thread.
 //
 // A hash chain is serial, and a lone GPU thread takes 0.87 us a block (64 dependent rounds at 27 cycles); a CPU core with the SHA
-// instructions takes about 0.04 us, one without them about 0.25.  So a caller's transcript that absorbs a long vector which the
+// instructions takes 0.05 us, one without them 0.3.  So a caller's transcript that absorbs a long vector which the
 // call has on the host (the scores and outputs of a row attention proof: read from it, or written into it) absorbs it here: its
 // 112-byte state is fetched, advanced and put back in stream order.
 #pragma once

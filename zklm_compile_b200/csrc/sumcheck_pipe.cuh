@@ -3,8 +3,8 @@
 // (rust/zk_ml_prover/src/proving/sumcheck.rs:211-272, 1262-1315 compute the same messages).
 //
 // In the plain tail every round is: pass over the tables (fold with the last challenge, sum the
-// round polynomial), block reduction, then one thread hashes (about five SHA-256 compressions)
-// while a thousand threads wait.  Here warp 0 only hashes.  While it hashes round k, the other warps
+// round polynomial), block reduction, then one warp hashes (about five SHA-256 compressions, a second warp beside it)
+// while thirty wait.  Here warp 0 only hashes.  While it hashes round k, the other warps
 // fold the tables with r_(k-1) and compute the NEXT round's sums as polynomials in the still
 // unknown r_k: with lo(r) = a + r (b - a), hi(r) = c + r (d - c) over the four quarters a, b, c,
 // d of a table, each of s0 = sum lo_f lo_g, s1 = sum hi_f hi_g, s2 = sum (2hi - lo)_f (2hi - lo)_g

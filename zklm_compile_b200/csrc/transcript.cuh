@@ -329,7 +329,10 @@ __device__ __noinline__ Sha8 sha256_compress_chain(Sha8 hin, const unsigned char
     o.v[4] = hin.v[4] + e; o.v[5] = hin.v[5] + f; o.v[6] = hin.v[6] + g; o.v[7] = hin.v[7] + h;
     return o;
 }
-// The second warp's part, all lanes: serves compressions until tr_pair_end.  Two words a step: even lanes the even schedule
+// The second warp's part, all lanes: serves compressions until tr_pair_end.  A kernel that uses a pair is launched with two whole
+// warps at least (the chains and the verifiers' kernels with exactly 64 threads), both of which reach their part: the hand-overs
+// are barriers of 64 threads, at which a lone warp would wait for good.
+//  Two words a step: even lanes the even schedule
 // words, odd lanes the odd ones.  With x[j] = W[2j + l] and z[j] = W[2j - 1 + l] (words of the other lane) a step is
 // x[j] = sig1(x[j-1]) + z[j-3] + sig0(z[j-7]) + x[j-8].
 __device__ __forceinline__ u32 sha_sig0(u32 v) { return sha_xor3(rotr32(v, 7), rotr32(v, 18), v >> 3); }

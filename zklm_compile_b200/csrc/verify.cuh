@@ -5,7 +5,7 @@
 // array plus one descriptor per (round, tree).  Three kernels then run:
 //
 //   bf_verify_chain_kernel   the transcript of all rounds (challenge, root absorb, 24 query squeezes
-//                            each): one thread, the same serial SHA-256 chain the prover runs
+//                            each): a pair of warps, the same serial SHA-256 chain the prover runs
 //   bf_verify_batch_kernel   one CTA per (round, tree): leaves sorted and de-duplicated, then level by
 //                            level the missing siblings merged in from the proof and the parents
 //                            hashed in parallel, up to the root; does not depend on the transcript,

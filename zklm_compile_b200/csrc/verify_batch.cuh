@@ -4,7 +4,7 @@
 // The host decodes the bytes into the flat word array and the per-tree descriptors of verify.cuh; the Merkle checks of all
 // trees (two per round, the joined polynomials' trees, the individual openings) are one launch of bf_verify_batch_kernel on the
 // second stream, the transcript (roots, rho, batched root, fold point, per round alpha / root / 24 queries, the last 24 queries)
-// one thread on the main stream, and the fold relation with the joined polynomials' contributions one warp per (round, query).
+// a pair of warps on the main stream, and the fold relation with the joined polynomials' contributions one warp per (round, query).
 // Like the reference's verifier it reads neither the final value nor the commitments' num_coeffs.
 #pragma once
 #include "verify.cuh"
