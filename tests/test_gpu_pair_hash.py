@@ -55,3 +55,25 @@ def test_attention_transcript_at_the_host_absorb_line(ctx, heads, seq, d):
         t2 = zk.Transcript(ctx, label)
         assert attention.verify_row_attention(proof, k, v, heads, seq, d, t2)
         assert t.squeeze_ef().tolist() == o.squeeze_ef().tolist() == t2.squeeze_ef().tolist()
+
+
+def test_op_list_whose_attention_streams_the_host_absorbs(ctx):
+    """Two attention ops of 2560 and 2760 words, behind and in front of other ops of the same transcript; a second proof on the same list."""
+    from zklm_compile_b200 import oplist, tables
+    rng = np.random.default_rng(9)
+    table = tables.build_exp_table(100)
+    small = lambda n: np.mod(rng.integers(-1, 2, n), P).astype(np.uint32)
+    shapes = [(2, 32, 8), (3, 23, 17)]
+    x = small(int(np.prod(shapes[0])))
+    g, o = oplist.OpList(ctx, len(x)), O.OpList()
+    for i, (h, s, d) in enumerate(shapes):
+        n = h * s * d
+        if i:
+            q = small(n)
+            g.set_input("in", q); o.set_input("in", q)
+        k, v = small(n), rng.integers(0, P, n, dtype=np.int64).astype(np.uint32)
+        g.attention("attn%d" % i, h, s, d, ctx.upload(table), k, v); o.attention("attn%d" % i, h, s, d, table, k, v)
+        w = rng.integers(0, P, (5 + i, n), dtype=np.int64).astype(np.uint32)
+        g.linear("out%d" % i, w, None, 5 + i, n); o.linear("out%d" % i, w, None, 5 + i, n)
+    want = o.prove(x)
+    assert g.prove(x) == want and g.prove(x) == want
